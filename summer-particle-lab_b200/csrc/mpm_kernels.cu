@@ -510,31 +510,32 @@ void launch_sort_scatter(const Ctx& c, cudaStream_t st, bool initial) {
 //   kPassG2P2G  gather -> F update -> advect -> return map -> scatter of the new state
 //   kPassG2P    gather -> F update -> advect -> return map (no scatter; host round-trip steps)
 // Scatter in two phases per tile (up to kCap particles per round):
-//   A  thread per particle: compute the new state and a 22-float payload (fraction t, m, m v,
+//   A  thread per particle: compute the new state and a 23-float payload (fraction t, m, m v,
 //      m C h, -4V/h tau); bucket it by its stencil base inside the 8^3 scatter window
 //      (shared-memory counting sort, native integer atomics)
 //   B  thread per (non-empty base bucket, z layer): all particles of a bucket hit the same 27
-//      nodes, so the 9 nodes x 7 channels of one layer are summed in registers and written with
-//      63 shared atomics per bucket and layer (about 24 per particle instead of 189)
+//      nodes, so the 9 nodes x 7 channels of one layer are summed in registers and added to the
+//      window without atomics (phase_b)
 // then one float4 atomic per touched node and channel group flushes the window to HBM.
 
 // Particles per scatter round. A full tile holds 512 (64 cells x 8), but a block that drifts by a
-// fraction of a cell leaves a third of its tiles a few particles over 512 (up to ~530); at
-// kCap = 512 those took a second round (every phase and barrier again for a handful of particles).
-constexpr int kCap = 768;
+// fraction of a cell leaves a third of its tiles a few particles over 512 (up to ~530); at a cap of
+// 512 those took a second round (every phase and barrier again for a handful of particles). 608 is
+// what two CTAs per SM leave beside the window copies.
+constexpr int kCap = 608;
+constexpr int kWinCopyNodes = 6 * kWinS * kWinS;  // nodes of one window copy: six bucket layers
 constexpr int kPf = 2;         // perm entries of the next tile's first round held per thread (shared memory)
-// Payload of one particle: 12 float pairs, laid out for the paired FMAs of phase B:
-//   0 (tx, ty)   1 (tz, m)    2 (mv0, mv1)  3 (mv2, m T)  [m T only with conduction, else 0]
-//   4 (c02, c12) 5 (c22, s02) 6 (s12, s22)  7 (c01, c11)  8 (c21, s01)  9 (c00, c10)  10 (c20, s00)
-//   11 (s11, 0)
+// Payload of one particle: six float4 rows laid out for the paired FMAs of phase B:
+//   0 (tx, ty, tz, m)       1 (mv0, mv1, mv2, m T)  [m T only with conduction, else 0]
+//   2 (c02, c12, c22, s02)  3 (s12, s22, c01, c11)  4 (c21, s01, c00, c10)  5 (c20, s00, s11, s12)
 // with c = m h C and s = -4 V / h tau (symmetric).
-constexpr int kPayRows = 12;
+constexpr int kPayRows = 6;
 constexpr int kBuckets = 216;  // 6^3 possible stencil bases in the scatter window
-// Payload slot of particle j: one extra word every 32 slots, so the slots phase B reads at a
-// stride of a bucket's size (8 for the particles of one cell in consecutive slots) fall in
-// different shared-memory banks; phase A's consecutive slots stay conflict-free.
-constexpr int kPayStride = kCap + kCap / 32;
-__device__ __forceinline__ int pay_slot(int j) { return j + (j >> 5); }
+// Payload slot of particle j: the slots phase B reads at a stride of a bucket's size (8 for the
+// particles of one cell in consecutive slots) fall in different shared-memory banks; phase A's
+// eight consecutive slots stay within one 128-byte line.
+__device__ __forceinline__ int pay_slot(int j) { return j ^ ((j >> 3) & 7); }
+static_assert(kCap % 8 == 0, "pay_slot permutes within blocks of eight");
 constexpr unsigned kMetaInvalid = 0x80000000u;
 
 enum Pass : int { kPassP2G = 0, kPassG2P2G = 1, kPassG2P = 2 };
@@ -548,13 +549,14 @@ struct TileCtx {
   long long node_base;
   float H, invH;
   int clamp;
-  int mat;  // material row of a single-material scene
+  int mat;   // material row of a single-material scene
+  float dt;  // the scene's substep
 };
 
 struct __align__(128) PartSmem {
   float4 vwin[2][kWinG * kWinG * kWinG];  // double-buffered TMA destinations (3456 B each)
-  float acc[kChannels * kWinSNodes];      // 16 KiB scatter window
-  float2 pay[kPayRows * kPayStride];      // 74 KiB payloads, structure of pair arrays (swizzled slots)
+  float4 win[3][2][kWinCopyNodes];        // 36 KiB scatter window (see win_node)
+  float4 pay[kPayRows * kCap];            // 57 KiB payloads, structure of float4 arrays (swizzled slots)
   unsigned meta[kCap];                    // bucket | rank << 8 (or kMetaInvalid)
   unsigned short sidx[kCap];              // slots sorted by bucket
   int hist[kBuckets];
@@ -565,23 +567,21 @@ struct __align__(128) PartSmem {
   unsigned long long mbar[2];
   uint4 item[2];
   int abort_flag;
-  unsigned red[3 * (kBlock / 32)];
+  unsigned red[3];   // the tile's CFL maxima (float bits) and status flags
   unsigned gate[2];  // learned mode: returns the gate accepted / sent to the bisection
   // State the CTA carries from tile to tile sits here rather than in registers: at 128 registers a
   // thread, every register held across the tiles is one fewer for phase A, and moving these (with
   // the heat sum, which was a per-thread double) cut the pass by 7%.
   unsigned tma_phase[2];       // mbarrier phases of the two window buffers (thread 0)
   double work_sum;             // heat from plastic work of the CTA's particles
-  int mt_row;                  // material row held in mt
-  int pf_ok;                   // pfs holds the next tile's first-round perm entries
   unsigned pfs[kPf * kBlock];  // perm entries j of the next tile's first round, j < kPf x kBlock
 
-  TileCtx tc;
+  TileCtx tc[2];               // by item buffer
   MaterialDev mt;
 };
 
 size_t particle_smem_bytes() { return sizeof(PartSmem); }
-static_assert(sizeof(PartSmem) <= 112 * 1024, "two CTAs per SM");
+static_assert(sizeof(PartSmem) <= 113 * 1024, "two CTAs per SM");
 
 // Direct global scatter (rare: particles that left the window, pinned particles): 27 nodes x
 // channel atomics straight to the accumulators, and the node tiles they touch become active.
@@ -612,6 +612,14 @@ __device__ __noinline__ void scatter_global(const Ctx& c, const SceneDev& sc, co
   mark_node_tiles_of(c, sc, b[0], b[1], b[2], nxt);
 }
 
+// Marks node tile tid of the 27 that a tile's scatter window covers as active.
+__device__ __forceinline__ void mark_window(const Ctx& c, const SceneDev& sc, int nxt, const int tile[3], int tid) {
+  const int dx = tid % 3 - 1, dy = (tid / 3) % 3 - 1, dz = tid / 9 - 1;
+  const int tx = tile[0] + dx, ty = tile[1] + dy, tz = tile[2] + dz;
+  if (tx >= 0 && ty >= 0 && tz >= 0 && tx < sc.ntiles[0] && ty < sc.ntiles[1] && tz < sc.ntiles[2])
+    mark_node_tile(c, sc.node_tile_base + (tz * sc.ntiles[1] + ty) * sc.ntiles[0] + tx, nxt);
+}
+
 // Flush the shared scatter window of one tile to the global accumulators (one float4 atomic per
 // touched node and channel group) and clear it; mark the 27 node tiles it covers as active.
 // tid / nthreads: this thread's index among the threads that flush.
@@ -637,43 +645,47 @@ __device__ __forceinline__ void flush_window_p(const Ctx& c, const SceneDev& sc,
 #pragma unroll
     for (int ch = 0; ch < kChannels; ++ch) acc[ch * kWinSNodes + i] = 0.f;
   }
-  if (tid < 27) {
-    const int dx = tid % 3 - 1, dy = (tid / 3) % 3 - 1, dz = tid / 9 - 1;
-    const int tx = tile[0] + dx, ty = tile[1] + dy, tz = tile[2] + dz;
-    if (tx >= 0 && ty >= 0 && tz >= 0 && tx < sc.ntiles[0] && ty < sc.ntiles[1] && tz < sc.ntiles[2])
-      mark_node_tile(c, sc.node_tile_base + (tz * sc.ntiles[1] + ty) * sc.ntiles[0] + tx, nxt);
-  }
+  if (tid < 27) mark_window(c, sc, nxt, tile, tid);
 }
 
+// The scatter window of the default pass: one copy per z layer kz of the stencil, indexed by the
+// bucket's z (node z = lz + kz), each node (m, p0, p1, p2) and (f0, f1, f2, m T) in two planes. Odd rows
+// are rotated by four nodes, so the eight lanes of a 128-bit access (four buckets of two rows) fall in
+// different banks.
+__device__ __forceinline__ int win_node(int lz, int y, int x) {
+  return (lz * kWinS + y) * kWinS + ((x + 4 * (y & 1)) & (kWinS - 1));
+}
+
+// The same for the default pass: sums the window's copies of each node and clears them.
 __device__ __forceinline__ void flush_window(const Ctx& c, const SceneDev& sc, PartSmem& sm, int nxt,
                                              const int tile[3]) {
-  flush_window_p(c, sc, sm.acc, nxt, tile, threadIdx.x, kBlock);
-}
-
-// Block reduction of the per-thread CFL maxima and status flags of one tile, then one atomic per
-// tile and scene. Every thread of the CTA calls it.
-__device__ __forceinline__ void block_reduce_item(const Ctx& c, int scene, float wave, float grad, unsigned flags,
-                                                  unsigned* red) {
-  const unsigned wb = __reduce_max_sync(0xffffffffu, fbits(wave));
-  const unsigned gb = __reduce_max_sync(0xffffffffu, fbits(grad));
-  const unsigned fl = __reduce_or_sync(0xffffffffu, flags);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) {
-    red[wid * 3 + 0] = wb;
-    red[wid * 3 + 1] = gb;
-    red[wid * 3 + 2] = fl;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned w = 0, g = 0, f = 0;
-    for (int k = 0; k < kBlock / 32; ++k) {
-      w = max(w, red[k * 3 + 0]);
-      g = max(g, red[k * 3 + 1]);
-      f |= red[k * 3 + 2];
+  const int o0 = tile[0] * kTile - 1, o1 = tile[1] * kTile - 1, o2 = tile[2] * kTile - 1;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int i = threadIdx.x; i < kWinSNodes; i += kBlock) {
+    const int lx = i & 7, ly = (i >> 3) & 7, lz = i >> 6;
+    float4 u = zero, v = zero;
+#pragma unroll
+    for (int kz = 0; kz < 3; ++kz) {
+      const int l = lz - kz;
+      if (l < 0 || l > 5) continue;
+      float4* A = &sm.win[kz][0][win_node(l, ly, lx)];
+      const float4 a = A[0], b = A[kWinCopyNodes];
+      u.x += a.x; u.y += a.y; u.z += a.z; u.w += a.w;
+      v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
+      A[0] = zero;
+      A[kWinCopyNodes] = zero;
     }
-    atomicMax(&c.wave_max[scene], w);
-    atomicMax(&c.grad_max[scene], g);
-    if (f) atomicOr(&c.ctrl->status, f);
+    if (u.x != 0.f) {
+      const int x = o0 + lx, y = o1 + ly, z = o2 + lz;
+      if (x >= 0 && y >= 0 && z >= 0) {
+        const long long node = sc.node_base + ((long long)z * sc.gdim[1] + y) * sc.gdim[0] + x;
+        atomicAdd(&c.g.acc0[nxt][node], u);
+        // the fourth channel of the second group is pinned mass in the grid (pinned particles
+        // scatter globally); the window's is the heat sum w m T, with conduction
+        atomicAdd(&c.g.acc1[nxt][node], make_float4(v.x, v.y, v.z, 0.f));
+        if (c.conduct) atomicAdd(&c.g.heat[nxt][node], v.w);
+      }
+    }
   }
 }
 
@@ -687,102 +699,135 @@ __device__ __forceinline__ unsigned state_flags(const float v[3], const float D[
   return f;
 }
 
-// Phase B task: one non-empty base bucket, one z layer of its stencil. Sums the 3x3 nodes x 7
-// channels over the bucket's particles in registers, then adds them to the shared window. The
-// channels run as one scalar (mass) and three pairs (p0, p1), (p2, f0), (f1, f2) of paired FMAs.
+// Quadratic B-spline weight of node k (0, 1, 2) at distance d = t - k; k need not be a constant.
+__device__ __forceinline__ float bspline_weight(int k, float d) {
+  const float a = 1.5f - fabsf(d);
+  return k == 1 ? fmaf(-d, d, 0.75f) : 0.5f * a * a;
+}
+
+// Phase B task: one non-empty base bucket, one z layer of its stencil. The 3x3 nodes x 7 channels (8
+// with conduction) are summed over the bucket's particles in registers. The channels run as one
+// scalar (mass) and three pairs (p0, p1), (p2, f0), (f1, f2) of paired FMAs.
 template <bool HEAT>
-__device__ __forceinline__ void bucket_layer_p(const float2* pay, const unsigned short* sidx, const int* bstart,
-                                               float* acc, int b, int kz) {
-  const int lx = b % 6, ly = (b / 6) % 6, lz = b / 36;
-  float a0[3][3];
+struct LayerSum {
+  float m[3][3], heat[3][3];
   float2 a12[3][3], a34[3][3], a56[3][3];
+};
+
+template <bool HEAT>
+__device__ __forceinline__ void sum_layer(const float4* pay, const unsigned short* sidx, int i0, int i1, int kz,
+                                          LayerSum<HEAT>& s) {
 #pragma unroll
   for (int y = 0; y < 3; ++y)
 #pragma unroll
     for (int x = 0; x < 3; ++x) {
-      a0[y][x] = 0.f;
-      a12[y][x] = a34[y][x] = a56[y][x] = dup2(0.f);
+      s.m[y][x] = s.heat[y][x] = 0.f;
+      s.a12[y][x] = s.a34[y][x] = s.a56[y][x] = dup2(0.f);
     }
-  const int i1 = bstart[b + 1];
-  for (int i = bstart[b]; i < i1; ++i) {
-    const int j = sidx[i];
-    const float2* P = pay + pay_slot(j);
-    const float2 txy = P[0 * kPayStride], tzm = P[1 * kPayStride], mv01 = P[2 * kPayStride];
-    const float2 mv2h = P[3 * kPayStride], E = P[4 * kPayStride], Fz = P[5 * kPayStride];
-    const float2 G = P[6 * kPayStride], H = P[7 * kPayStride], I = P[8 * kPayStride];
-    const float2 K = P[9 * kPayStride], L = P[10 * kPayStride], S11 = P[11 * kPayStride];
-    const float2 J = make_float2(S11.x, G.x);  // (s11, s12)
-    const float2 M = make_float2(I.y, Fz.y);   // (s01, s02)
-    float wx[3], wy[3], wzv[3];
-    bspline_weights(txy.x, wx);
-    bspline_weights(txy.y, wy);
-    bspline_weights(tzm.x, wzv);
-    const float wz = kz == 0 ? wzv[0] : (kz == 1 ? wzv[1] : wzv[2]);
-    const float2 dz2 = dup2(static_cast<float>(kz) - tzm.x);
-    const float2 q01 = ffma2(E, dz2, mv01);                        // (mv0 + c02 dz, mv1 + c12 dz)
-    const float2 q2g0 = ffma2(Fz, dz2, make_float2(mv2h.x, 0.f));  // (mv2 + c22 dz, s02 dz)
-    const float2 g12 = fmul2(G, dz2);                              // (s12 dz, s22 dz)
-    const float mwz = tzm.y * wz;
+#pragma unroll 1
+  for (int i = i0; i < i1; ++i) {
+    const float4* P = pay + pay_slot(sidx[i]);
+    const float4 r0 = P[0 * kCap], r1 = P[1 * kCap], r2 = P[2 * kCap], r3 = P[3 * kCap], r4 = P[4 * kCap],
+                 r5 = P[5 * kCap];
+    float wx[3], wy[3];
+    bspline_weights(r0.x, wx);
+    bspline_weights(r0.y, wy);
+    const float ez = r0.z - static_cast<float>(kz);
+    const float wz = bspline_weight(kz, ez);
+    const float2 dz2 = dup2(-ez);
+    const float2 q01 = ffma2(make_float2(r2.x, r2.y), dz2, make_float2(r1.x, r1.y));
+    const float2 q2g0 = ffma2(make_float2(r2.z, r2.w), dz2, make_float2(r1.z, 0.f));
+    const float2 g12 = fmul2(make_float2(r3.x, r3.y), dz2);
+    const float2 K = make_float2(r4.z, r4.w), L = make_float2(r5.x, r5.y), M = make_float2(r4.y, r2.w);
 #pragma unroll
     for (int y = 0; y < 3; ++y) {
-      const float2 dy2 = dup2(static_cast<float>(y) - txy.y);
+      const float2 dy2 = dup2(static_cast<float>(y) - r0.y);
       const float wyz = wy[y] * wz;
-      const float2 p01 = ffma2(H, dy2, q01), p2f0 = ffma2(I, dy2, q2g0), f12 = ffma2(J, dy2, g12);
-      const float mwyz = mwz * wy[y];
+      const float2 p01 = ffma2(make_float2(r3.z, r3.w), dy2, q01), p2f0 = ffma2(make_float2(r4.x, r4.y), dy2, q2g0),
+                   f12 = ffma2(make_float2(r5.z, r5.w), dy2, g12);
+      const float mw = r0.w * wyz, hw = r1.w * wyz;
 #pragma unroll
       for (int x = 0; x < 3; ++x) {
-        const float2 dx2 = dup2(static_cast<float>(x) - txy.x);
+        const float2 dx2 = dup2(static_cast<float>(x) - r0.x);
         const float2 wt = dup2(wx[x] * wyz);
-        a0[y][x] = fmaf(wx[x], mwyz, a0[y][x]);
-        a12[y][x] = ffma2(wt, ffma2(K, dx2, p01), a12[y][x]);
-        a34[y][x] = ffma2(wt, ffma2(L, dx2, p2f0), a34[y][x]);
-        a56[y][x] = ffma2(wt, ffma2(M, dx2, f12), a56[y][x]);
+        s.m[y][x] = fmaf(wx[x], mw, s.m[y][x]);
+        if (HEAT) s.heat[y][x] = fmaf(wx[x], hw, s.heat[y][x]);  // sum w m T (conduction)
+        s.a12[y][x] = ffma2(wt, ffma2(K, dx2, p01), s.a12[y][x]);
+        s.a34[y][x] = ffma2(wt, ffma2(L, dx2, p2f0), s.a34[y][x]);
+        s.a56[y][x] = ffma2(wt, ffma2(M, dx2, f12), s.a56[y][x]);
       }
     }
   }
+}
+
+// The warp-specialised pass adds a task's sums to its window with shared atomics.
+template <bool HEAT>
+__device__ __forceinline__ void bucket_layer_p(const float4* pay, const unsigned short* sidx, const int* bstart,
+                                               float* acc, int b, int kz) {
+  const int lx = b % 6, ly = (b / 6) % 6, lz = b / 36;
+  LayerSum<HEAT> s;
+  sum_layer<HEAT>(pay, sidx, bstart[b], bstart[b + 1], kz, s);
 #pragma unroll
   for (int y = 0; y < 3; ++y)
 #pragma unroll
     for (int x = 0; x < 3; ++x) {
       float* A = acc + ((lz + kz) * kWinS + (ly + y)) * kWinS + (lx + x);
-      atomicAdd(A + 0 * kWinSNodes, a0[y][x]);
-      atomicAdd(A + 1 * kWinSNodes, a12[y][x].x);
-      atomicAdd(A + 2 * kWinSNodes, a12[y][x].y);
-      atomicAdd(A + 3 * kWinSNodes, a34[y][x].x);
-      atomicAdd(A + 4 * kWinSNodes, a34[y][x].y);
-      atomicAdd(A + 5 * kWinSNodes, a56[y][x].x);
-      atomicAdd(A + 6 * kWinSNodes, a56[y][x].y);
+      atomicAdd(A + 0 * kWinSNodes, s.m[y][x]);
+      atomicAdd(A + 1 * kWinSNodes, s.a12[y][x].x);
+      atomicAdd(A + 2 * kWinSNodes, s.a12[y][x].y);
+      atomicAdd(A + 3 * kWinSNodes, s.a34[y][x].x);
+      atomicAdd(A + 4 * kWinSNodes, s.a34[y][x].y);
+      atomicAdd(A + 5 * kWinSNodes, s.a56[y][x].x);
+      atomicAdd(A + 6 * kWinSNodes, s.a56[y][x].y);
+      if (HEAT) atomicAdd(A + 7 * kWinSNodes, s.heat[y][x]);
     }
-  if (HEAT) {  // sum w m T into channel 7 (conduction)
-    float hsum[3][3];
-#pragma unroll
-    for (int y = 0; y < 3; ++y)
-#pragma unroll
-      for (int x = 0; x < 3; ++x) hsum[y][x] = 0.f;
-    for (int i = bstart[b]; i < i1; ++i) {
-      const float2* P = pay + pay_slot(sidx[i]);
-      const float2 txy = P[0 * kPayStride];
-      float wx[3], wy[3], wzv[3];
-      bspline_weights(txy.x, wx);
-      bspline_weights(txy.y, wy);
-      bspline_weights(P[1 * kPayStride].x, wzv);
-      const float wmt = (kz == 0 ? wzv[0] : (kz == 1 ? wzv[1] : wzv[2])) * P[3 * kPayStride].y;
-#pragma unroll
-      for (int y = 0; y < 3; ++y)
-#pragma unroll
-        for (int x = 0; x < 3; ++x) hsum[y][x] += wx[x] * wy[y] * wmt;
-    }
-#pragma unroll
-    for (int y = 0; y < 3; ++y)
-#pragma unroll
-      for (int x = 0; x < 3; ++x)
-        atomicAdd(&acc[7 * kWinSNodes + ((lz + kz) * kWinS + (ly + y)) * kWinS + (lx + x)], hsum[y][x]);
-  }
 }
 
+// Phase B of the default pass: one thread per (non-empty bucket, z layer kz) sums its nine nodes, then
+// nine steps add them to the window copy of kz, one node offset (y, x) a step. Tasks of one copy
+// have different buckets, so in one step they touch different nodes and plain 128-bit loads and stores
+// do; CTA barriers separate the steps. Shared fp32 atomics in their place are retry loops of about 120 cycles each,
+// 63 in a row per thread: they held phase B at 17.5k of a full tile's 46k cycles (2M-particle block, two
+// CTAs per SM), the steps at 12.1k of 32.8k; the whole pass went from 0.357 to 0.289 ms. Threads without a
+// task sum an empty range: a branch around the sums cost 250 bytes of spills in phase A, as did
+// letting the compiler unroll the loops that hold the 63 sums. Ends at a barrier.
 template <bool HEAT>
-__device__ __forceinline__ void bucket_layer(PartSmem& sm, int b, int kz) {
-  bucket_layer_p<HEAT>(sm.pay, sm.sidx, sm.bstart, sm.acc, b, kz);
+__device__ __forceinline__ void phase_b(PartSmem& sm, int nbk) {
+  const int ntasks = 3 * nbk;
+#pragma unroll 1
+  for (int t0 = 0; t0 == 0 || t0 < ntasks; t0 += kBlock) {  // one round at least: the caller counts on its barriers
+    const int task = t0 + static_cast<int>(threadIdx.x);
+    const bool has = task < ntasks;
+    const int kz = has ? task / nbk : 0;
+    const int b = has ? sm.blist[task - kz * nbk] : 0;
+    const int i0 = has ? sm.bstart[b] : 0, i1 = has ? sm.bstart[b + 1] : 0;
+    LayerSum<HEAT> s;
+    sum_layer<HEAT>(sm.pay, sm.sidx, i0, i1, kz, s);
+    const int lx = b % 6, ly = (b / 6) % 6, lz = b / 36;
+#pragma unroll
+    for (int y = 0; y < 3; ++y) {
+      float4* row = &sm.win[kz][0][(lz * kWinS + ly + y) * kWinS];
+      const int rot = lx + 4 * ((ly + y) & 1);
+#pragma unroll
+      for (int x = 0; x < 3; ++x) {
+        if (has) {
+          float4* A = row + ((rot + x) & (kWinS - 1));
+          float4 u = A[0], v = A[kWinCopyNodes];
+          u.x += s.m[y][x];
+          u.y += s.a12[y][x].x;
+          u.z += s.a12[y][x].y;
+          u.w += s.a34[y][x].x;
+          v.x += s.a34[y][x].y;
+          v.y += s.a56[y][x].x;
+          v.z += s.a56[y][x].y;
+          if (HEAT) v.w += s.heat[y][x];
+          A[0] = u;
+          A[kWinCopyNodes] = v;
+        }
+        __syncthreads();
+      }
+    }
+  }
 }
 
 // Exclusive scan of the bucket histogram over a group of NT >= kBuckets threads, with the compact
@@ -917,7 +962,7 @@ __device__ __noinline__ Gather12 gather_global(const float4* base, int sy, long 
 template <int PASS, bool HEAT, bool AUX, bool NEWTON = false>
 __device__ __forceinline__ unsigned particle_phase_a(const Ctx& c, const SceneDev& sc, const TileCtx& tc,
                                                      const MaterialDev& mt_single, bool single, const float4* vwin,
-                                                     unsigned home, unsigned j, float dt, int nxt, float2* pay,
+                                                     unsigned home, unsigned j, float dt, int nxt, float4* pay,
                                                      unsigned* meta, int* hist, float& wave_acc, float& grad_acc,
                                                      unsigned& flags_acc, double& work_acc, bool store_vc,
                                                      unsigned* gate = nullptr) {
@@ -1100,19 +1145,13 @@ __device__ __forceinline__ unsigned particle_phase_a(const Ctx& c, const SceneDe
       if (lane == leader) rank0 = atomicAdd(&hist[bucket], __popc(peers));
       const int rank = __shfl_sync(peers, rank0, leader) + __popc(peers & ((1u << lane) - 1u));
       meta[j] = static_cast<unsigned>(bucket) | (static_cast<unsigned>(rank) << 8);
-      float2* P = pay + pay_slot(j);
-      P[0 * kPayStride] = make_float2(t[0], t[1]);
-      P[1 * kPayStride] = make_float2(t[2], m);
-      P[2 * kPayStride] = make_float2(mv[0], mv[1]);
-      P[3 * kPayStride] = make_float2(mv[2], HEAT ? m * T : 0.f);
-      P[4 * kPayStride] = make_float2(mC[2], mC[5]);
-      P[5 * kPayStride] = make_float2(mC[8], s6[4]);
-      P[6 * kPayStride] = make_float2(s6[5], s6[2]);
-      P[7 * kPayStride] = make_float2(mC[1], mC[4]);
-      P[8 * kPayStride] = make_float2(mC[7], s6[3]);
-      P[9 * kPayStride] = make_float2(mC[0], mC[3]);
-      P[10 * kPayStride] = make_float2(mC[6], s6[0]);
-      P[11 * kPayStride] = make_float2(s6[1], 0.f);
+      float4* P = pay + pay_slot(j);
+      P[0 * kCap] = make_float4(t[0], t[1], t[2], m);
+      P[1 * kCap] = make_float4(mv[0], mv[1], mv[2], HEAT ? m * T : 0.f);
+      P[2 * kCap] = make_float4(mC[2], mC[5], mC[8], s6[4]);
+      P[3 * kCap] = make_float4(s6[5], s6[2], mC[1], mC[4]);
+      P[4 * kCap] = make_float4(mC[7], s6[3], mC[0], mC[3]);
+      P[5 * kCap] = make_float4(mC[6], s6[0], s6[1], s6[5]);
     } else {
       meta[j] = kMetaInvalid;
       if (!in_w) flags |= 0x10u;
@@ -1180,7 +1219,7 @@ template <int PASS>
 __device__ __forceinline__ unsigned particle_phase_a_learned(const Ctx& c, const SceneDev& sc, const TileCtx& tc,
                                                              const MaterialDev& mt_single, bool single,
                                                              const float4* vwin, bool live, unsigned home, unsigned j,
-                                                             float dt, int nxt, float2* pay, unsigned* meta, int* hist,
+                                                             float dt, int nxt, float4* pay, unsigned* meta, int* hist,
                                                              float& wave_acc, float& grad_acc, unsigned& flags_acc,
                                                              double& work_acc, bool store_vc, unsigned* gate) {
   constexpr bool SCATTER = PASS != kPassG2P;
@@ -1330,19 +1369,13 @@ __device__ __forceinline__ unsigned particle_phase_a_learned(const Ctx& c, const
       if (lane == leader) rank0 = atomicAdd(&hist[bucket], __popc(peers));
       const int rank = __shfl_sync(peers, rank0, leader) + __popc(peers & ((1u << lane) - 1u));
       meta[j] = static_cast<unsigned>(bucket) | (static_cast<unsigned>(rank) << 8);
-      float2* P = pay + pay_slot(j);
-      P[0 * kPayStride] = make_float2(t[0], t[1]);
-      P[1 * kPayStride] = make_float2(t[2], m);
-      P[2 * kPayStride] = make_float2(mv[0], mv[1]);
-      P[3 * kPayStride] = make_float2(mv[2], 0.f);
-      P[4 * kPayStride] = make_float2(mC[2], mC[5]);
-      P[5 * kPayStride] = make_float2(mC[8], s6[4]);
-      P[6 * kPayStride] = make_float2(s6[5], s6[2]);
-      P[7 * kPayStride] = make_float2(mC[1], mC[4]);
-      P[8 * kPayStride] = make_float2(mC[7], s6[3]);
-      P[9 * kPayStride] = make_float2(mC[0], mC[3]);
-      P[10 * kPayStride] = make_float2(mC[6], s6[0]);
-      P[11 * kPayStride] = make_float2(s6[1], 0.f);
+      float4* P = pay + pay_slot(j);
+      P[0 * kCap] = make_float4(t[0], t[1], t[2], m);
+      P[1 * kCap] = make_float4(mv[0], mv[1], mv[2], 0.f);
+      P[2 * kCap] = make_float4(mC[2], mC[5], mC[8], s6[4]);
+      P[3 * kCap] = make_float4(s6[5], s6[2], mC[1], mC[4]);
+      P[4 * kCap] = make_float4(mC[7], s6[3], mC[0], mC[3]);
+      P[5 * kCap] = make_float4(mC[6], s6[0], s6[1], s6[5]);
     } else {
       meta[j] = kMetaInvalid;
       if (!in_w) flags |= 0x10u;
@@ -1413,6 +1446,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_particles(const __grid_constant__
   PartSmem& sm = *reinterpret_cast<PartSmem*>(smem_raw);
   constexpr bool SCATTER = PASS != kPassG2P;
   constexpr bool GATHER = PASS != kPassP2G;
+  constexpr unsigned kNone = 0xffffffffu;
   Ctrl* ct = c.ctrl;
   if (PASS == kPassG2P2G && blockIdx.x == 0 && threadIdx.x == 0) {  // for the sort that follows
     ct->sort_list = ct->step_index & 1u;
@@ -1426,8 +1460,87 @@ __global__ void __launch_bounds__(kBlock, 2) k_particles(const __grid_constant__
   const int lst = PASS == kPassP2G ? (k & 1) : ((k - 1) & 1);
   const int nxt = k & 1;
   const bool use_tma = GATHER && c.use_tma;
+  const bool single = c.single_material != 0 || c.scene_material != 0;
+
+  // One thread claims a work item for buffer `buf`: item, tile constants, the velocity window's TMA
+  // and the L2 prefetch of the tile's particles.
+  auto claim = [&](int buf) {
+    const unsigned idx = atomicAdd(&ct->work_next, 1u);
+    const uint4 nx = idx < ct->work_count[lst] ? c.s.work[lst][idx] : make_uint4(kNone, 0, 0, 0);
+    sm.item[buf] = nx;
+    if (nx.x == kNone) return;
+    const SceneDev& sc = c.scenes[nx.w];
+    TileCtx& tl = sm.tc[buf];
+    const int lt = static_cast<int>(nx.x) - sc.tile_base;
+    const int tx = lt % sc.tiles[0], ty = (lt / sc.tiles[0]) % sc.tiles[1], tz = lt / (sc.tiles[0] * sc.tiles[1]);
+    if (use_tma && !sm.abort_flag) {
+      fence_proxy_async_smem();
+      mbar_arrive_expect_tx(&sm.mbar[buf], sizeof(sm.vwin[0]));
+      tma_load_4d(sm.vwin[buf], static_cast<const char*>(c.tmaps) + 128 * nx.w, 0, tx * kTile, ty * kTile, tz * kTile,
+                  &sm.mbar[buf]);
+    }
+    tl.tile[0] = tx;
+    tl.tile[1] = ty;
+    tl.tile[2] = tz;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      tl.dims[a] = sc.dims[a];
+      tl.gdim[a] = sc.gdim[a];
+      tl.qlo[a] = sc.qlo[a];
+      tl.qhi[a] = sc.qhi[a];
+    }
+    tl.node_base = sc.node_base;
+    tl.H = sc.H;
+    tl.invH = sc.invH;
+    tl.clamp = sc.clamp;
+    tl.mat = sc.mat_base;
+    tl.dt = GATHER ? c.dt_scene[nx.w] : 0.f;
+    prefetch_tile_state<AUX>(c, nx);
+  };
+  // Every thread of the CTA, between two tiles: what the next tile (buffer buf, already claimed) needs
+  // before phase A, in the shadow of the previous tile's flush.
+  unsigned pf[kPf];
+  auto load_perm = [&](int buf) {
+    const uint4 nx = sm.item[buf];
+#pragma unroll
+    for (int q = 0; q < kPf; ++q) {
+      const unsigned j = q * kBlock + threadIdx.x;
+      pf[q] = nx.x != kNone && j < nx.z ? c.p.perm[nx.y + j] : 0u;
+    }
+  };
+  auto finish_next = [&](int buf, int mat_now) {
+#pragma unroll
+    for (int q = 0; q < kPf; ++q) sm.pfs[q * kBlock + threadIdx.x] = pf[q];
+    if (sm.item[buf].x == kNone) return;
+    // the material row of a single-material handle or of the tile's scene in a batch, only when it
+    // changes (every tile of a one-scene handle shares it; a batch's tiles come scene by scene)
+    if (single && sm.tc[buf].mat != mat_now) {
+      static_assert(sizeof(MaterialDev) % 4 == 0, "word copy");
+      const unsigned* src = reinterpret_cast<const unsigned*>(c.mats + sm.tc[buf].mat);
+      unsigned* dst = reinterpret_cast<unsigned*>(&sm.mt);
+      for (int i = threadIdx.x; i < static_cast<int>(sizeof(MaterialDev) / 4); i += kBlock) dst[i] = src[i];
+    }
+    if (GATHER && !use_tma) {
+      const TileCtx& tl = sm.tc[buf];
+      for (int i = threadIdx.x; i < kWinG * kWinG * kWinG; i += kBlock) {
+        const int x = tl.tile[0] * kTile + i % kWinG, y = tl.tile[1] * kTile + (i / kWinG) % kWinG,
+                  z = tl.tile[2] * kTile + i / (kWinG * kWinG);
+        sm.vwin[buf][i] = c.g.vel[tl.node_base + ((long long)z * tl.gdim[1] + y) * tl.gdim[0] + x];
+      }
+    }
+    if (use_tma && threadIdx.x == 0) {
+      const unsigned ph = sm.tma_phase[buf];
+      if (!mbar_wait_bounded(&sm.mbar[buf], ph)) {
+        atomicOr(&ct->status, 0x8u);
+        mbar_wait_bounded(&sm.mbar[buf], ph);  // a second bounded chance for the copy in flight
+        sm.abort_flag = 1;
+      }
+      sm.tma_phase[buf] ^= 1u;
+    }
+  };
+
   if (SCATTER) {
-    for (int i = threadIdx.x; i < kChannels * kWinSNodes; i += kBlock) sm.acc[i] = 0.f;
+    for (int i = threadIdx.x; i < 3 * 2 * kWinCopyNodes; i += kBlock) (&sm.win[0][0][0])[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int i = threadIdx.x; i < kBuckets; i += kBlock) sm.hist[i] = 0;
   }
   if (threadIdx.x == 0) {
@@ -1438,129 +1551,54 @@ __global__ void __launch_bounds__(kBlock, 2) k_particles(const __grid_constant__
     sm.gate[0] = sm.gate[1] = 0u;
     sm.tma_phase[0] = sm.tma_phase[1] = 0u;
     sm.work_sum = 0.0;
-    sm.mt_row = -1;
-    sm.pf_ok = 0;
-    const unsigned idx = atomicAdd(&ct->work_next, 1u);
-    sm.item[0] = idx < ct->work_count[lst] ? c.s.work[lst][idx] : make_uint4(0xffffffffu, 0, 0, 0);
-    if (use_tma && sm.item[0].x != 0xffffffffu) {
-      const uint4 it = sm.item[0];
-      const SceneDev& sc = c.scenes[it.w];
-      const int lt = static_cast<int>(it.x) - sc.tile_base;
-      mbar_arrive_expect_tx(&sm.mbar[0], sizeof(sm.vwin[0]));
-      tma_load_4d(sm.vwin[0], static_cast<const char*>(c.tmaps) + 128 * it.w, 0, (lt % sc.tiles[0]) * kTile,
-                  ((lt / sc.tiles[0]) % sc.tiles[1]) * kTile, (lt / (sc.tiles[0] * sc.tiles[1])) * kTile, &sm.mbar[0]);
-    }
+    sm.red[0] = sm.red[1] = sm.red[2] = 0u;
+    claim(0);
   }
-  int cb = 0;
-  while (true) {
-    __syncthreads();
-    const uint4 it = sm.item[cb];
-    if (it.x == 0xffffffffu) break;
-    if (threadIdx.x == 0) {
-      if (use_tma) {
-        const unsigned ph = sm.tma_phase[cb];
-        if (!mbar_wait_bounded(&sm.mbar[cb], ph)) {
-          atomicOr(&ct->status, 0x8u);
-          mbar_wait_bounded(&sm.mbar[cb], ph);  // a second bounded chance for the copy in flight
-          sm.abort_flag = 1;
-        }
-        sm.tma_phase[cb] ^= 1u;
-      }
-    }
-    // The next work item is claimed, and its velocity window requested, by thread 0 after phase A
-    // of this tile's first round, so the two dependent global round trips overlap other warps' work.
-    auto prefetch_next = [&]() {
-      const unsigned idx = atomicAdd(&ct->work_next, 1u);
-      const uint4 nx = idx < ct->work_count[lst] ? c.s.work[lst][idx] : make_uint4(0xffffffffu, 0, 0, 0);
-      sm.item[cb ^ 1] = nx;
-      if (use_tma && nx.x != 0xffffffffu && !sm.abort_flag) {
-        const SceneDev& sn = c.scenes[nx.w];
-        const int lt = static_cast<int>(nx.x) - sn.tile_base;
-        fence_proxy_async_smem();
-        mbar_arrive_expect_tx(&sm.mbar[cb ^ 1], sizeof(sm.vwin[0]));
-        tma_load_4d(sm.vwin[cb ^ 1], static_cast<const char*>(c.tmaps) + 128 * nx.w, 0, (lt % sn.tiles[0]) * kTile,
-                    ((lt / sn.tiles[0]) % sn.tiles[1]) * kTile, (lt / (sn.tiles[0] * sn.tiles[1])) * kTile,
-                    &sm.mbar[cb ^ 1]);
-      }
-      if (nx.x != 0xffffffffu) prefetch_tile_state<AUX>(c, nx);
-    };
-    const int scene = static_cast<int>(it.w);
-    const SceneDev& sc = c.scenes[scene];
-    if (threadIdx.x == 0) {  // per-tile constants, computed once and read from shared memory
-      TileCtx tl;
-      const int lt = static_cast<int>(it.x) - sc.tile_base;
-      tl.tile[0] = lt % sc.tiles[0];
-      tl.tile[1] = (lt / sc.tiles[0]) % sc.tiles[1];
-      tl.tile[2] = lt / (sc.tiles[0] * sc.tiles[1]);
-#pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        tl.dims[a] = sc.dims[a];
-        tl.gdim[a] = sc.gdim[a];
-        tl.qlo[a] = sc.qlo[a];
-        tl.qhi[a] = sc.qhi[a];
-      }
-      tl.node_base = sc.node_base;
-      tl.H = sc.H;
-      tl.invH = sc.invH;
-      tl.clamp = sc.clamp;
-      tl.mat = sc.mat_base;
-      sm.tc = tl;
-    }
-    // the material row of a single-material handle or of the tile's scene in a batch, copied word
-    // by word by the whole block, and only when it changes (every tile of a one-scene handle shares
-    // it; a batch's tiles come scene by scene)
-    const int mt_row = sm.mt_row;
-    if ((c.single_material || c.scene_material) && sc.mat_base != mt_row) {
-      static_assert(sizeof(MaterialDev) % 4 == 0, "word copy");
-      const unsigned* src = reinterpret_cast<const unsigned*>(c.mats + sc.mat_base);
-      unsigned* dst = reinterpret_cast<unsigned*>(&sm.mt);
-      for (int i = threadIdx.x; i < static_cast<int>(sizeof(MaterialDev) / 4); i += kBlock) dst[i] = src[i];
-      __syncthreads();
-      if (threadIdx.x == 0) sm.mt_row = sc.mat_base;
-    }
-    __syncthreads();
+  __syncthreads();
+  load_perm(0);
+  finish_next(0, -1);
+  __syncthreads();
+  for (int cb = 0;; cb ^= 1) {
+    if (sm.item[cb].x == kNone) break;
     if (sm.abort_flag) return;
-    if (GATHER && !use_tma) {
-      const TileCtx& tl = sm.tc;
-      for (int i = threadIdx.x; i < kWinG * kWinG * kWinG; i += kBlock) {
-        const int x = tl.tile[0] * kTile + i % kWinG, y = tl.tile[1] * kTile + (i / kWinG) % kWinG,
-                  z = tl.tile[2] * kTile + i / (kWinG * kWinG);
-        sm.vwin[cb][i] = c.g.vel[tl.node_base + ((long long)z * tl.gdim[1] + y) * tl.gdim[0] + x];
-      }
-      __syncthreads();
-    }
-    const TileCtx& tc = sm.tc;
-    const float dt = GATHER ? c.dt_scene[scene] : 0.f;
-    const bool single = c.single_material != 0 || c.scene_material != 0;
-    float wave_acc = 0.f, grad_acc = 0.f;
-    unsigned flags_acc = 0;
+    const TileCtx& tc = sm.tc[cb];
     for (unsigned r0 = 0; r0 < sm.item[cb].z; r0 += kCap) {
       const unsigned nround = min(static_cast<unsigned>(kCap), sm.item[cb].z - r0);
       // ---- phase A: one thread per particle (the bucket histogram is zero: cleared at the start
       // and by each round's scan) ----
       for (unsigned jj = 0; jj < nround; jj += kBlock) {
         const unsigned j = jj + threadIdx.x;
-        unsigned key = 0xffffffffu;
+        if (jj + (threadIdx.x & ~31u) >= nround) break;  // warps past the end of the round
+        const bool live = j < nround;
+        unsigned key = kNone;
+        float wave = 0.f, grad = 0.f;
+        unsigned flags = 0;
+        const SceneDev& sc = c.scenes[sm.item[cb].w];
         if constexpr (JC == 1) {
-          // every lane of a warp with a live particle takes part in its network evaluation (warps
-          // past the end of the round skip as a whole)
-          if (jj + (threadIdx.x & ~31u) >= nround) continue;
-          const bool live = j < nround;
-          const unsigned home = !live ? c.p.perm[it.y + r0]
-                                      : (r0 == 0 && sm.pf_ok && jj < kPf * kBlock) ? sm.pfs[jj + threadIdx.x]
-                                                                                 : c.p.perm[it.y + r0 + j];
-          key = particle_phase_a_learned<PASS>(c, sc, tc, sm.mt, single, sm.vwin[cb], live, home, j, dt, nxt, sm.pay,
-                                               sm.meta, sm.hist, wave_acc, grad_acc, flags_acc, sm.work_sum, store_vc,
-                                               sm.gate);
-        } else if (j < nround) {
-          const unsigned home = (r0 == 0 && sm.pf_ok && jj < kPf * kBlock) ? sm.pfs[jj + threadIdx.x] : c.p.perm[sm.item[cb].y + r0 + j];
-          key = particle_phase_a<PASS, HEAT, AUX, JC == 2>(c, sc, tc, sm.mt, single, sm.vwin[cb], home, j, dt, nxt,
-                                                           sm.pay, sm.meta, sm.hist, wave_acc, grad_acc, flags_acc,
-                                                           sm.work_sum, store_vc, sm.gate);
+          // every lane of a warp with a live particle takes part in its network evaluation
+          const unsigned home = !live ? c.p.perm[sm.item[cb].y + r0]
+                                      : (r0 == 0 && jj < kPf * kBlock) ? sm.pfs[j] : c.p.perm[sm.item[cb].y + r0 + j];
+          key = particle_phase_a_learned<PASS>(c, sc, tc, sm.mt, single, sm.vwin[cb], live, home, j, tc.dt, nxt, sm.pay,
+                                               sm.meta, sm.hist, wave, grad, flags, sm.work_sum, store_vc, sm.gate);
+        } else if (live) {
+          const unsigned home = (r0 == 0 && jj < kPf * kBlock) ? sm.pfs[j] : c.p.perm[sm.item[cb].y + r0 + j];
+          key = particle_phase_a<PASS, HEAT, AUX, JC == 2>(c, sc, tc, sm.mt, single, sm.vwin[cb], home, j, tc.dt, nxt,
+                                                           sm.pay, sm.meta, sm.hist, wave, grad, flags, sm.work_sum,
+                                                           store_vc, sm.gate);
         }
         if (PASS == kPassG2P2G) count_key(c, key);
+        // CFL maxima and status flags of the tile
+        const unsigned wb = __reduce_max_sync(0xffffffffu, fbits(wave));
+        const unsigned gb = __reduce_max_sync(0xffffffffu, fbits(grad));
+        const unsigned fl = __reduce_or_sync(0xffffffffu, flags);
+        if ((threadIdx.x & 31) == 0) {
+          atomicMax(&sm.red[0], wb);
+          atomicMax(&sm.red[1], gb);
+          if (fl) atomicOr(&sm.red[2], fl);
+        }
       }
-      if (!SCATTER && r0 == 0 && threadIdx.x == 0) prefetch_next();
+      // the last thread claims the next tile (a full tile has about 3 x 64 phase-B tasks, so its warp
+      // rarely has one), another warp marks this tile's node tiles
       if (SCATTER) {
         __syncthreads();
         scan_buckets(sm);
@@ -1570,33 +1608,28 @@ __global__ void __launch_bounds__(kBlock, 2) k_particles(const __grid_constant__
           if (!(mm & kMetaInvalid)) sm.sidx[sm.bstart[mm & 0xffu] + (mm >> 8)] = static_cast<unsigned short>(j);
         }
         __syncthreads();
-        // ---- phase B: one thread per (non-empty bucket, z layer); the last thread claims the next
-        // tile meanwhile (a full tile has about 3 x 64 tasks, so it rarely has one)
-        if (r0 == 0 && threadIdx.x == kBlock - 1) prefetch_next();
-        const int nbk = sm.nbuckets;
-        for (int task = threadIdx.x; task < 3 * nbk; task += kBlock) {
-          const int kz = task / nbk;
-          bucket_layer<HEAT>(sm, sm.blist[task - kz * nbk], kz);
+        if (r0 == 0) {
+          if (threadIdx.x == kBlock - 1) claim(cb ^ 1);
+          const int lane27 = static_cast<int>(threadIdx.x) - (kBlock - 64);
+          if (lane27 >= 0 && lane27 < 27) mark_window(c, c.scenes[sm.item[cb].w], nxt, tc.tile, lane27);
         }
-        __syncthreads();
-        if (r0 == 0) {  // perm of the next tile's first round, consumed there
-          const uint4 nx = sm.item[cb ^ 1];
-          const bool ok = nx.x != 0xffffffffu;
-          if (threadIdx.x == 0) sm.pf_ok = ok;
-          if (ok) {
-#pragma unroll
-            for (int k = 0; k < kPf; ++k) {
-              const unsigned j = k * kBlock + threadIdx.x;
-              sm.pfs[j] = j < nx.z ? c.p.perm[nx.y + j] : 0u;
-            }
-          }
-        }
+        phase_b<HEAT>(sm, sm.nbuckets);  // ends at a barrier
+      } else if (r0 == 0) {
+        if (threadIdx.x == kBlock - 1) claim(cb ^ 1);
       }
     }
-    block_reduce_item(c, scene, wave_acc, grad_acc, flags_acc, sm.red);
+    if (!SCATTER) __syncthreads();
+    load_perm(cb ^ 1);
+    if (threadIdx.x == 32) {
+      const unsigned scene = sm.item[cb].w;
+      atomicMax(&c.wave_max[scene], sm.red[0]);
+      atomicMax(&c.grad_max[scene], sm.red[1]);
+      if (sm.red[2]) atomicOr(&ct->status, sm.red[2]);
+      sm.red[0] = sm.red[1] = sm.red[2] = 0u;
+    }
+    if (SCATTER) flush_window(c, c.scenes[sm.item[cb].w], sm, nxt, tc.tile);
+    finish_next(cb ^ 1, tc.mat);
     __syncthreads();
-    if (SCATTER) flush_window(c, sc, sm, nxt, tc.tile);
-    cb ^= 1;
   }
   if (JC != 0 && threadIdx.x == 0) {  // gate counts: one atomic each per CTA (the loop ended at a barrier)
     if (sm.gate[0]) atomicAdd(&c.gate_counts[0], sm.gate[0]);
@@ -1631,7 +1664,7 @@ struct StageInfo {
 
 struct __align__(128) WsSmem {
   float4 vwin[2][kWinG * kWinG * kWinG];  // producer: double-buffered TMA destinations
-  float2 pay[2][kPayRows * kPayStride];   // stage buffers
+  float4 pay[2][kPayRows * kCap];         // stage buffers
   unsigned meta[2][kCap];
   int hist[2][kBuckets];
   StageInfo info[2];
