@@ -1083,36 +1083,60 @@ int mpm_stable_dt(mpm_handle* h, double* dt) {
   return MPM_OK;
 }
 
-// Lays out the regularisation scratch for the current scenes and spacing: neighbour cells two
-// spacings wide over each scene's grid, the cell sort and the per-particle shifts.
-static int ensure_regularizer(mpm_handle* h) {
-  if (!h->reg_dirty && h->rblock) return MPM_OK;
-  const double hc = 2 * h->reg.spacing;
+// Neighbour cells of width hc over every scene's grid: fills rs, returns the total or -1 above 2^30.
+static long long layout_cells(const mpm_handle* h, double hc, std::vector<mpm::RegScene>& rs) {
   const int ns = static_cast<int>(h->scenes.size());
-  std::vector<mpm::RegScene> rs(ns);
+  rs.assign(ns, mpm::RegScene{});
   long long cells = 0;
   for (int s = 0; s < ns; ++s) {
     const SceneDev& sc = h->scenes[s];
-    long long k = 1;
+    double k = 1;
     for (int a = 0; a < 3; ++a) {
       const double ext = (sc.dims[a] - 1) * static_cast<double>(sc.H);
       rs[s].nc[a] = static_cast<int>(std::min(1.0e9, std::floor(ext / hc))) + 1;
       k *= rs[s].nc[a];
     }
     rs[s].cell_base = cells;
-    cells += k;
-    if (cells > (1ll << 30)) return fail(h, MPM_ERR_INVALID_ARG, "regularisation spacing too small for the grid");
+    if (k > static_cast<double>((1ll << 30) - cells)) return -1;
+    cells += static_cast<long long>(k);
   }
+  return cells;
+}
+
+// The finer of two cell widths unless its cells outnumber the particles eightfold (a mostly empty grid:
+// the counts' clear and scan would cost more than the shorter candidate lists save), then the coarser;
+// the coarser decides what is refused.
+static long long choose_cells(const mpm_handle* h, double fine, double coarse, std::vector<mpm::RegScene>& rs, double* hc) {
+  const long long most = layout_cells(h, coarse, rs);
+  *hc = coarse;
+  if (most < 0) return -1;
+  std::vector<mpm::RegScene> rf;
+  const long long cells = layout_cells(h, fine, rf);
+  if (cells < 0 || cells > std::max<long long>(8 * h->cap, 1 << 20)) return most;
+  rs.swap(rf);
+  *hc = fine;
+  return cells;
+}
+
+// Lays out the regularisation scratch for the current scenes and spacing: neighbour cells one spacing
+// (or two, see choose_cells) wide over each scene's grid, the cell sort and the per-particle shifts.
+static int ensure_regularizer(mpm_handle* h) {
+  if (!h->reg_dirty && h->rblock) return MPM_OK;
+  const int ns = static_cast<int>(h->scenes.size());
+  std::vector<mpm::RegScene> rs;
+  double hc = 0;
+  const long long cells = choose_cells(h, h->reg.spacing, 2 * h->reg.spacing, rs, &hc);
+  if (cells < 0) return fail(h, MPM_ERR_INVALID_ARG, "regularisation spacing too small for the grid");
   const int64_t cap = h->cap;
   const size_t nb = mpm::reg_scan_blocks(cells);
   auto lay = [&](char* base, mpm::RegBufs& b, mpm::RegScene** scenes) {
     Carver cv{base};
     *scenes = cv.take<mpm::RegScene>(ns);
-    b.count = cv.take<unsigned>(cells);
-    b.start = cv.take<unsigned>(cells);
-    b.cursor = cv.take<unsigned>(cells);
+    b.count = cv.take<unsigned>(cells + 1);
+    b.start = cv.take<unsigned>(cells + 1);
     b.block_sums = cv.take<unsigned>(nb + 1);
-    b.largest = cv.take<unsigned>(ns);
+    b.largest = cv.take<unsigned>(2 * ns);
+    b.tmax = b.largest ? b.largest + ns : nullptr;
     b.cell_of = cv.take<unsigned>(cap);
     b.sorted = cv.take<unsigned>(cap);
     b.target = cv.take<float>(cap);
@@ -1134,6 +1158,7 @@ static int ensure_regularizer(mpm_handle* h) {
   }
   h->rblock_bytes = bytes;
   lay(static_cast<char*>(h->rblock), h->rbufs, &sp);
+  MPM_CUDA(h, cudaMemsetAsync(h->rbufs.count, 0, sizeof(unsigned) * (cells + 1), h->stream));
   MPM_CUDA(h, cudaMemcpyAsync(sp, rs.data(), sizeof(mpm::RegScene) * ns, cudaMemcpyHostToDevice, h->stream));
   MPM_CUDA(h, cudaStreamSynchronize(h->stream));  // rs is a host temporary
   mpm::RegDev& r = h->rdev;
@@ -1144,6 +1169,7 @@ static int ensure_regularizer(mpm_handle* h) {
   r.max_speed = static_cast<float>(h->reg.max_speed);
   r.rate = static_cast<float>(h->reg.rate);
   r.eps = static_cast<float>(h->reg.spacing * 1e-8 / 2.8);  // 1e-8 in the reference's units (spacing 2.8)
+  r.hc = static_cast<float>(hc);
   r.inv_hc = static_cast<float>(1.0 / hc);
   h->reg_dirty = false;
   return MPM_OK;
@@ -1435,28 +1461,17 @@ int mpm_regularize(mpm_handle* h, double dt) {
 static int ensure_heat(mpm_handle* h, double radius) {
   if (h->hblock && h->heat_radius == radius) return MPM_OK;
   const int ns = static_cast<int>(h->scenes.size());
-  std::vector<mpm::RegScene> rs(ns);
-  long long cells = 0;
-  for (int s = 0; s < ns; ++s) {
-    const SceneDev& sc = h->scenes[s];
-    long long k = 1;
-    for (int a = 0; a < 3; ++a) {
-      const double ext = (sc.dims[a] - 1) * static_cast<double>(sc.H);
-      rs[s].nc[a] = static_cast<int>(std::min(1.0e9, std::floor(ext / radius))) + 1;
-      k *= rs[s].nc[a];
-    }
-    rs[s].cell_base = cells;
-    cells += k;
-    if (cells > (1ll << 30)) return fail(h, MPM_ERR_INVALID_ARG, "heat-exchange radius too small for the grid");
-  }
+  std::vector<mpm::RegScene> rs;
+  double hc = 0;
+  const long long cells = choose_cells(h, radius / 2, radius, rs, &hc);
+  if (cells < 0) return fail(h, MPM_ERR_INVALID_ARG, "heat-exchange radius too small for the grid");
   const int64_t cap = h->cap;
   const size_t nb = mpm::reg_scan_blocks(cells);
   auto lay = [&](char* base, mpm::HeatBufs& b, mpm::RegScene** scenes) {
     Carver cv{base};
     *scenes = cv.take<mpm::RegScene>(ns);
-    b.count = cv.take<unsigned>(cells);
-    b.start = cv.take<unsigned>(cells);
-    b.cursor = cv.take<unsigned>(cells);
+    b.count = cv.take<unsigned>(cells + 1);
+    b.start = cv.take<unsigned>(cells + 1);
     b.block_sums = cv.take<unsigned>(nb + 1);
     b.exchanged = cv.take<double>(1);
     b.cell_of = cv.take<unsigned>(cap);
@@ -1482,10 +1497,13 @@ static int ensure_heat(mpm_handle* h, double radius) {
   }
   h->hblock_bytes = bytes;
   lay(static_cast<char*>(h->hblock), h->hbufs, &sp);
+  MPM_CUDA(h, cudaMemsetAsync(h->hbufs.count, 0, sizeof(unsigned) * (cells + 1), h->stream));
   MPM_CUDA(h, cudaMemcpyAsync(sp, rs.data(), sizeof(mpm::RegScene) * ns, cudaMemcpyHostToDevice, h->stream));
   MPM_CUDA(h, cudaStreamSynchronize(h->stream));  // rs is a host temporary
   h->hdev.scenes = sp;
   h->hdev.cells = cells;
+  h->hdev.hc = static_cast<float>(hc);
+  h->hdev.inv_hc = static_cast<float>(1.0 / hc);
   h->heat_radius = radius;
   return MPM_OK;
 }
@@ -1501,7 +1519,6 @@ int mpm_exchange_heat(mpm_handle* h, const mpm_heat_exchange* x, double dt, doub
   int rc = ensure_heat(h, x->radius);
   if (rc != MPM_OK) return rc;
   mpm::HeatDev hd = h->hdev;
-  hd.inv_hc = static_cast<float>(1.0 / x->radius);
   hd.radius = static_cast<float>(x->radius);
   hd.eps = static_cast<float>(x->radius * 1.25e-7);  // 1e-6 of the reference's 8-unit radius
   hd.geom_rate = static_cast<float>(x->geometry * x->heat_rate);

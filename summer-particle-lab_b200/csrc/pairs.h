@@ -22,13 +22,15 @@ struct RegDev {
   float max_speed;        // displacement budget per second (m/s)
   float rate;             // gain = 1 - exp(-rate dt)
   float eps;              // coincident pairs: r < eps
-  float inv_hc;           // 1 / neighbour cell size (cells are two spacings wide)
+  float hc, inv_hc;       // neighbour cell size (see ensure_regularizer) and its inverse
   const float* dt_scene;  // per-scene dt of the substep just taken, or null: dt
   float dt;
 };
 
 struct RegBufs {
-  unsigned *cell_of, *count, *start, *cursor, *sorted, *block_sums, *largest;
+  // count: particles per cell, zero between passes; start: cells + 1 entries; largest and tmax: per scene
+  // (float bits, contiguous), the largest shift over its budget and the largest target spacing
+  unsigned *cell_of, *count, *start, *sorted, *block_sums, *largest, *tmax;
   float *target, *inv_mass;
   float4* shift;
   uint4* pos_sorted;             // cell order: (qx, qy, qz, target bits)
@@ -39,12 +41,12 @@ struct RegBufs {
 size_t reg_scan_blocks(long long cells);
 void launch_regularize(const Ctx& c, const RegDev& r, const RegBufs& b, cudaStream_t st);
 
-// Particle-pair heat exchange: neighbour cells one radius wide (RegScene layout), conductance
-// factor geometry * heat_rate, optional ambient loss.
+// Particle-pair heat exchange: neighbour cells (RegScene layout), conductance factor geometry *
+// heat_rate, optional ambient loss.
 struct HeatDev {
   const RegScene* scenes;
   long long cells;
-  float inv_hc;         // 1 / radius
+  float hc, inv_hc;     // neighbour cell size (see ensure_heat) and its inverse
   float radius, eps;    // pairs with eps < r < radius
   float geom_rate;      // geometry * heat_rate
   float dt;
@@ -53,7 +55,7 @@ struct HeatDev {
 };
 
 struct HeatBufs {
-  unsigned *cell_of, *count, *start, *cursor, *sorted, *block_sums;
+  unsigned *cell_of, *count, *start, *sorted, *block_sums;  // as in RegBufs
   uint4* pos_sorted;    // cell order: (qx, qy, qz, T bits)
   float2* prop_sorted;  // cell order: (conductivity, m cp)
   float* budget;        // cell order
