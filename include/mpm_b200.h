@@ -241,7 +241,8 @@ int mpm_grid_debug(mpm_handle* h, double dt, double* mass, double* momentum);
 
 /* Per-kernel device time, measured with CUDA events on the handle's stream around each launch
  * while enabled (reference: s.profile stage timers, src/three/mpm.js:60-133).
- * Kernel ids: 0 begin, 1 grid update, 2 g2p2g, 3 scan, 4 sort scatter, 5 p2g, 6 keys. */
+ * Kernel ids: 0 begin, 1 grid update, 2 g2p2g, 3 scan, 4 sort scatter, 5 p2g, 6 keys. Within a call a
+ * substep's launches under 0 and 1 also scan and sort when the pass before them asked for it. */
 #define MPM_PROFILE_KERNELS 7
 int mpm_profile_enable(mpm_handle* h, int32_t on);
 int mpm_profile_read(mpm_handle* h, double ms[MPM_PROFILE_KERNELS], int64_t launches[MPM_PROFILE_KERNELS]);

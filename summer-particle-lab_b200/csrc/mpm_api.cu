@@ -60,11 +60,7 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 struct mpm_handle {
   std::string err;
   cudaStream_t stream = nullptr;
-  // The tile sort after a scatter pass runs on `side` beside the next substep's k_begin and grid
-  // update; `main_ev` orders it after the pass, `side_ev` orders the next pass after it.
-  cudaStream_t side = nullptr;
-  cudaEvent_t main_ev = nullptr, side_ev = nullptr;
-  bool side_pending = false;
+  bool sort_pending = false;  // the last scatter pass's keys are not sorted yet (the next grid launch sorts them)
   int num_sms = 148;
   mpm_domain dom{};
   SceneDev scene{};                  // scene 0 (the only scene of a single-scene handle)
@@ -104,7 +100,7 @@ struct mpm_handle {
   mpm::Ctrl* host_ctrl = nullptr;                        // pinned readback
   double* host_ledger = nullptr;                         // pinned readback
   Ctx ctx{};
-  int g2p2g_blocks = 0, p2g_blocks = 0, grid_blocks = 0;
+  int g2p2g_blocks = 0, p2g_blocks = 0, grid_blocks = 0, sort_blocks = 0;
   int ws_blocks = 0;  // warp-specialised scatter passes available (CTAs), 0: not available
   // solid position regularisation: parameters and scratch (cells, sort, shifts), built on use
   mpm_regularizer reg{};
@@ -290,16 +286,19 @@ static size_t carve_particles(char* base, int64_t cap, mpm::Particles& p) {
   return align_up(c.off, 256);
 }
 
-// Permutation pass: rewrite the state in sort order into the other buffer and make it current.
-// The main stream waits for a tile sort still running on the side stream.
-static void join_side(mpm_handle* h) {
-  if (!h->side_pending) return;
-  cudaStreamWaitEvent(h->stream, h->side_ev, 0);
-  h->side_pending = false;
+// Sorts the last scatter pass's keys now, where no grid update follows that would do it.
+static void finish_sort(mpm_handle* h) {
+  if (!h->sort_pending) return;
+  { ProfScope ps(h, 3); mpm::launch_open(h->ctx, h->stream, false, true); }
+  ProfScope ps(h, 4);
+  mpm::launch_grid_sort(h->ctx, h->stream, 0, h->sort_blocks);
+  h->sort_pending = false;
 }
 
+// Permutation pass: rewrite the state in sort order into the other buffer and make it current.
+
 static int permute_state(mpm_handle* h) {
-  join_side(h);
+  finish_sort(h);
   h->ctx.n = h->n;
   mpm::launch_permute(h->ctx, h->palt, h->stream);
   MPM_CUDA(h, cudaGetLastError());
@@ -390,7 +389,7 @@ static int alloc_grid(mpm_handle* h) {
                               h->stream));
   MPM_CUDA(h, cudaMemcpyAsync(const_cast<mpm::MaterialExt*>(c.mats_ext), h->mats_ext.data(),
                               sizeof(mpm::MaterialExt) * kMaxMats, cudaMemcpyHostToDevice, h->stream));
-  // TMA descriptor of each scene's velocity grid: 4D {channel 4, x, y, z}, box {4, 6, 6, 6}, fp32.
+  // TMA descriptor of each scene's velocity grid: 3D {4 channels x x, y, z}, box {4 x 8, 8, 8}, fp32.
   // A scene's grid starts at a float4 node (16-byte aligned) and its strides are multiples of 16 B.
   c.tmaps = nullptr;
   c.use_tma = 0;
@@ -401,11 +400,11 @@ static int alloc_grid(mpm_handle* h) {
     for (int k = 0; k < ns && ok; ++k) {
       const SceneDev& s = h->scenes[k];
       std::memset(&maps[k], 0, sizeof(CUtensorMap));
-      cuuint64_t gdims[4] = {4, (cuuint64_t)s.gdim[0], (cuuint64_t)s.gdim[1], (cuuint64_t)s.gdim[2]};
-      cuuint64_t gstrides[3] = {16, 16ull * s.gdim[0], 16ull * s.gdim[0] * s.gdim[1]};
-      cuuint32_t box[4] = {4, mpm::kWinG, mpm::kWinG, mpm::kWinG};
-      cuuint32_t estr[4] = {1, 1, 1, 1};
-      CUresult r = encode(&maps[k], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, c.g.vel + s.node_base, gdims, gstrides, box, estr,
+      cuuint64_t gdims[3] = {4ull * s.gdim[0], (cuuint64_t)s.gdim[1], (cuuint64_t)s.gdim[2]};
+      cuuint64_t gstrides[2] = {16ull * s.gdim[0], 16ull * s.gdim[0] * s.gdim[1]};
+      cuuint32_t box[3] = {4 * mpm::kWinG, mpm::kWinG, mpm::kWinG};
+      cuuint32_t estr[3] = {1, 1, 1};
+      CUresult r = encode(&maps[k], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, c.g.vel + s.node_base, gdims, gstrides, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
       ok = r == CUDA_SUCCESS;
@@ -459,7 +458,7 @@ static int status_error(mpm_handle* h, unsigned st) {
 }
 
 static int check_status(mpm_handle* h) {
-  join_side(h);
+  finish_sort(h);
   MPM_CUDA(h, cudaMemcpyAsync(h->host_ctrl, h->ctx.ctrl, sizeof(mpm::Ctrl), cudaMemcpyDeviceToHost, h->stream));
   MPM_CUDA(h, cudaStreamSynchronize(h->stream));
   return status_error(h, h->host_ctrl->status);
@@ -467,7 +466,7 @@ static int check_status(mpm_handle* h) {
 
 // Counting sort of the current state by tile and the dt-free P2G into acc[step_index & 1].
 static int prepare_grid(mpm_handle* h) {
-  join_side(h);
+  h->sort_pending = false;  // everything is sorted anew (the counts are cleared below)
   Ctx& c = h->ctx;
   c.n = h->n;
   if (h->pending_grid) {
@@ -479,7 +478,7 @@ static int prepare_grid(mpm_handle* h) {
   MPM_CUDA(h, cudaMemsetAsync(c.s.count, 0, sizeof(unsigned) * (c.total_tiles + 1), h->stream));
   { ProfScope ps(h, 6); mpm::launch_keys(c, h->stream); }
   { ProfScope ps(h, 3); mpm::launch_scan(c, h->stream, true); }
-  { ProfScope ps(h, 4); mpm::launch_sort_scatter(c, h->stream, true); }
+  { ProfScope ps(h, 4); mpm::launch_sort_scatter(c, h->stream); }
   if (h->reorder_pending) {
     ProfScope ps(h, -1);
     const int rc = permute_state(h);
@@ -494,31 +493,22 @@ static int prepare_grid(mpm_handle* h) {
   return MPM_OK;
 }
 
-// One substep: k_begin and the grid update (beside the previous pass's tile sort, if that is still
-// running on the side stream), then the particle pass; a scatter pass forks its tile sort (scan +
-// counting sort of the keys it wrote) onto the side stream, where it overlaps the next substep's
-// k_begin and grid update. The two never touch the same data: the sort works on the keys, counts,
-// perm and the work list of the pass's parity, k_begin and the grid update on the control block's
-// step fields, the other list's counters and the grid.
+// One substep: the prologue (and the scan of the previous pass's tile counts), the grid update (and the
+// tile sort of its keys), the particle pass.
 static void launch_substep(mpm_handle* h, bool scatter) {
   Ctx& c = h->ctx;
-  { ProfScope ps(h, 0); mpm::launch_begin(c, h->stream); }
-  { ProfScope ps(h, 1); mpm::launch_grid_update(c, h->stream, h->grid_blocks); }
+  // a permutation that follows this substep takes a fresh sort
+  c.force_sort = h->reorder_interval > 0 && h->substeps_since_reorder + 1 >= h->reorder_interval ? 1 : 0;
+  { ProfScope ps(h, 0); mpm::launch_open(c, h->stream, true, h->sort_pending); }
+  { ProfScope ps(h, 1); mpm::launch_grid_sort(c, h->stream, h->grid_blocks, h->sort_pending ? h->sort_blocks : 0); }
+  h->sort_pending = false;
   if (c.conduct) {
     ProfScope ps(h, -1);
     mpm::launch_conduct(c, h->stream, h->grid_blocks);
   }
-  join_side(h);
   { ProfScope ps(h, 2); mpm::launch_g2p2g(c, h->stream, h->g2p2g_blocks, scatter); }
   if (scatter && h->slab_planes) { ProfScope ps(h, -1); mpm::launch_halo_sum(c, h->stream, h->slab_planes); }
-  if (scatter) {
-    cudaEventRecord(h->main_ev, h->stream);
-    cudaStreamWaitEvent(h->side, h->main_ev, 0);
-    { ProfScope ps(h, 3, h->side); mpm::launch_scan(c, h->side, false); }
-    { ProfScope ps(h, 4, h->side); mpm::launch_sort_scatter(c, h->side, false); }
-    cudaEventRecord(h->side_ev, h->side);
-    h->side_pending = true;
-  }
+  h->sort_pending = scatter;
 }
 
 MaterialDev mpm::material_to_device(const mpm_material& m) {
@@ -689,15 +679,6 @@ int mpm_create(const mpm_domain* domain, int64_t capacity, mpm_handle** out) {
     delete h;
     return MPM_ERR_CUDA;
   }
-  if (cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaEventCreateWithFlags(&h->main_ev, cudaEventDisableTiming) != cudaSuccess ||
-      cudaEventCreateWithFlags(&h->side_ev, cudaEventDisableTiming) != cudaSuccess) {
-    if (h->main_ev) cudaEventDestroy(h->main_ev);
-    if (h->side) cudaStreamDestroy(h->side);
-    cudaStreamDestroy(h->stream);
-    delete h;
-    return MPM_ERR_CUDA;
-  }
   h->dom = *domain;
   h->scene = s;
   h->scenes.assign(1, s);
@@ -711,9 +692,6 @@ int mpm_create(const mpm_domain* domain, int64_t capacity, mpm_handle** out) {
   const size_t pbytes = carve_particles(nullptr, capacity, p);
   auto bail = [&](int code) {
     free_device(h);
-    cudaEventDestroy(h->main_ev);
-    cudaEventDestroy(h->side_ev);
-    cudaStreamDestroy(h->side);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
     return code;
@@ -753,6 +731,7 @@ int mpm_create(const mpm_domain* domain, int64_t capacity, mpm_handle** out) {
   h->ctx.ws_blocks = std::getenv("MPM_B200_WS") ? h->ws_blocks : 0;
   h->p2g_blocks = h->num_sms * mpm::p2g_blocks_per_sm();
   h->grid_blocks = h->num_sms * 8;
+  h->sort_blocks = h->num_sms * 8;
   if (cudaStreamSynchronize(h->stream) != cudaSuccess) return bail(MPM_ERR_CUDA);
   *out = h;
   return MPM_OK;
@@ -760,15 +739,10 @@ int mpm_create(const mpm_domain* domain, int64_t capacity, mpm_handle** out) {
 
 int mpm_destroy(mpm_handle* h) {
   if (!h) return MPM_ERR_INVALID_ARG;
-  join_side(h);
   if (h->stream) cudaStreamSynchronize(h->stream);
-  if (h->side) cudaStreamSynchronize(h->side);
   for (cudaEvent_t e : h->ev_pool) cudaEventDestroy(e);
   drop_graph(h);
   free_device(h);
-  if (h->main_ev) cudaEventDestroy(h->main_ev);
-  if (h->side_ev) cudaEventDestroy(h->side_ev);
-  if (h->side) cudaStreamDestroy(h->side);
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
   return MPM_OK;
@@ -1275,7 +1249,7 @@ static int run_substeps(mpm_handle* h, int mode, double dt_req, int max_substeps
       }
     }
     launched += est;
-    join_side(h);
+    finish_sort(h);
     MPM_CUDA(h, cudaGetLastError());
     MPM_CUDA(h, cudaMemcpyAsync(h->host_ctrl, h->ctx.ctrl, sizeof(mpm::Ctrl), cudaMemcpyDeviceToHost, h->stream));
     MPM_CUDA(h, cudaStreamSynchronize(h->stream));
@@ -1679,7 +1653,6 @@ int mpm_profile_enable(mpm_handle* h, int32_t on) {
 int mpm_profile_read(mpm_handle* h, double ms[MPM_PROFILE_KERNELS], int64_t launches[MPM_PROFILE_KERNELS]) {
   if (!h || !ms || !launches) return MPM_ERR_INVALID_ARG;
   MPM_CUDA(h, cudaStreamSynchronize(h->stream));
-  MPM_CUDA(h, cudaStreamSynchronize(h->side));  // the sort kernels' events
   for (int k = 0; k < MPM_PROFILE_KERNELS; ++k) {
     ms[k] = 0;
     launches[k] = 0;
@@ -1698,7 +1671,7 @@ int mpm_check_bounded_wait(mpm_handle* h, int64_t limit_cycles, int32_t* timed_o
   if (!h || !timed_out) return MPM_ERR_INVALID_ARG;
   if (limit_cycles <= 0 || limit_cycles > (1ll << 33))
     return fail(h, MPM_ERR_INVALID_ARG, "limit_cycles must be in (0, 2^33]");
-  join_side(h);
+  finish_sort(h);
   unsigned* dev = nullptr;
   MPM_CUDA(h, cudaMalloc(&dev, sizeof(unsigned)));
   unsigned host = 0;
@@ -2011,7 +1984,7 @@ int mpm_gate_counts_read(mpm_handle* h, mpm_gate_counts* out, int32_t reset) {
   if (!h->mlp_block) return MPM_OK;
   unsigned* counts = h->ctx.gate_counts;
   unsigned hc[2] = {0, 0};
-  join_side(h);
+  finish_sort(h);
   MPM_CUDA(h, cudaMemcpyAsync(hc, counts, sizeof hc, cudaMemcpyDeviceToHost, h->stream));
   if (reset) MPM_CUDA(h, cudaMemsetAsync(counts, 0, sizeof hc, h->stream));
   MPM_CUDA(h, cudaStreamSynchronize(h->stream));
@@ -2230,7 +2203,7 @@ static int capture_graph(mpm_handle* h, int count) {
   const bool prof = h->profiling;
   h->profiling = false;
   const int64_t launches0 = h->launches;  // captured launches run on replay, not now
-  join_side(h);  // the graph starts with nothing pending on the side stream
+  finish_sort(h);  // the graph starts with nothing pending
   MPM_CUDA(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
   for (int i = 0; i < count; ++i) {
     launch_substep(h, true);
@@ -2239,7 +2212,7 @@ static int capture_graph(mpm_handle* h, int count) {
       permute_state(h);
     }
   }
-  join_side(h);  // and ends with the side stream joined back
+  finish_sort(h);  // and ends that way
   cudaGraph_t g = nullptr;
   cudaError_t e = cudaStreamEndCapture(h->stream, &g);
   h->profiling = prof;
@@ -2293,7 +2266,7 @@ int mpm_batch_run(mpm_handle* h, int32_t nsteps, int32_t use_graph) {
       const int rc = capture_graph(h, chunk);
       if (rc != MPM_OK) return rc;
     }
-    join_side(h);
+    finish_sort(h);
     while (left >= chunk) {
       MPM_CUDA(h, cudaGraphLaunch(h->graph, h->stream));
       h->launches += h->launches_per_graph;
@@ -2304,7 +2277,7 @@ int mpm_batch_run(mpm_handle* h, int32_t nsteps, int32_t use_graph) {
     const int rc = eager_substep(h);
     if (rc != MPM_OK) return rc;
   }
-  join_side(h);
+  finish_sort(h);
   MPM_CUDA(h, cudaGetLastError());
   h->pending_grid = true;
   return check_status(h);

@@ -31,13 +31,17 @@ constexpr int kFracBits = 22;
 constexpr float kFixedOne = 4194304.0f;        // 2^22
 constexpr float kInvFixedOne = 2.384185791015625e-07f;
 constexpr int kTile = 4;                         // tile edge (cells / nodes)
-constexpr int kWinG = 6;                         // gather window edge (nodes)
+constexpr int kWinG = 8;                         // gather window edge (nodes)
 constexpr int kWinS = 8;                         // scatter window edge (nodes)
 constexpr int kWinSNodes = kWinS * kWinS * kWinS;
 constexpr int kChannels = 8;                     // m, px, py, pz, fx, fy, fz, pinned mass
 constexpr int kBlock = 256;                      // threads per CTA in the particle kernels
 constexpr int kMaxScenes = 4096;
 constexpr int kMaxMaterials = 4096;
+
+// Largest tile count whose scan k_open does by itself (3 us per 4,096 tiles, in the few substeps that sort);
+// above it k_scan is launched, about 2 us in every substep.
+constexpr int kOpenScanTiles = 16384;
 
 enum StepMode : int { kModeFixed = 0, kModeRequested = 1, kModeCfl = 2 };
 
@@ -87,8 +91,12 @@ struct Ctrl {
   unsigned scan_ticket;
   int steps_left;        // requested-dt steps of this call still to start after the current one, + 1
   int step_substeps;     // substeps of the current requested-dt step
-  unsigned sort_list;    // work list the sort after a scatter pass appends to (written by that pass)
-  unsigned sort_active;  // 1 if that pass ran (the sort and scan skip a pass that returned at done)
+  unsigned sort_list;    // the newest work list: what a particle pass reads, and the sort after a scan writes
+  unsigned sort_active;  // 1 if the last scatter pass wrote keys to sort (the scan and sort do nothing otherwise)
+  unsigned sort_want;    // 1: the next scatter pass writes keys (set by the substep's prologue from the two below)
+  unsigned strays;       // particles that left the tile whose list holds them, as of the last scatter pass
+  unsigned far_strays;   // some of them a whole cell or more
+  unsigned in_place;     // perm is the identity: the state was permuted after the newest sort
   unsigned last_substep; // 1 when the current substep is the call's last (set by k_begin): only then
                          // does the fused pass store particle velocities and APIC matrices, which no
                          // later substep of the call reads
@@ -157,6 +165,7 @@ struct Ctx {
   int has_thermal;      // temperature array is read and written
   int has_plastic;      // plastic strain array is read and written
   int has_aux;          // aux array is read and written (a snow, sand or pressure material is set)
+  int force_sort;       // this scatter pass writes keys whatever sort_want says
   int use_tma;
   int ws_blocks;        // > 0: the particle passes that scatter run warp-specialised on this many CTAs
   int conduct;          // a scene conducts heat on the grid: heat channel, conduction pass, dT gather
@@ -195,13 +204,15 @@ void launch_control_init(const Ctx& c, cudaStream_t st);
 void launch_keys(const Ctx& c, cudaStream_t st);
 void launch_scan(const Ctx& c, cudaStream_t st, bool initial);
 void launch_wait_probe(cudaStream_t st, unsigned* out, long long limit);
-void launch_sort_scatter(const Ctx& c, cudaStream_t st, bool initial);
+void launch_sort_scatter(const Ctx& c, cudaStream_t st);
 void launch_p2g(const Ctx& c, cudaStream_t st, int grid_blocks);
 void launch_control_step(const Ctx& c, cudaStream_t st, int mode, double dt_req, int max_substeps, float dt_fixed,
                          int nsteps = 1);
-void launch_begin(const Ctx& c, cudaStream_t st);
+void launch_open(const Ctx& c, cudaStream_t st, bool begin, bool scan);
 void launch_grid_clear(const Ctx& c, cudaStream_t st, int grid_blocks);
-void launch_grid_update(const Ctx& c, cudaStream_t st, int grid_blocks);
+// The grid update (grid_blocks CTAs) and, beside it, the tile sort of the last scatter pass (sort_blocks CTAs); either
+// may be 0.
+void launch_grid_sort(const Ctx& c, cudaStream_t st, int grid_blocks, int sort_blocks);
 void launch_conduct(const Ctx& c, cudaStream_t st, int grid_blocks);
 // Slab decomposition along z: consecutive scenes share `planes` node planes; after a scatter both
 // copies of every shared node hold the sum (only in node tiles the scene has active).

@@ -1,15 +1,14 @@
 // CUDA kernels of the B200-native MLS-MPM solid step (sm_100a).
 //
-// One substep is five launches on one stream (all persistent or grid-stride, no host sync):
-//   k_begin        1 CTA: dt from the device-side CFL maxima, step bookkeeping, list resets
-//   k_grid_update  active node tiles only: v = (p + dt (f + m g)) / m, walls, sticky floor
-//   k_g2p2g        per particle tile: TMA-staged 6^3 velocity window -> gather v, C -> F update
+// One substep is three launches on one stream (no host sync):
+//   k_open         1 CTA: dt from the device-side CFL maxima, step bookkeeping, list resets; after a pass
+//                  that wrote sort keys, the scan of the tile counts
+//   k_grid_sort    active node tiles only: v = (p + dt (f + m g)) / m, walls, sticky floor; beside it, after
+//                  such a pass, the counting sort: perm[start + rank] = particle
+//   k_particles    per particle tile: TMA-staged 8^3 velocity window -> gather v, C -> F update
 //                  -> advect -> constitutive update / J2 return -> scatter m, p, f of the new
 //                  state into an 8^3 shared-memory window -> one float4 atomic per node per tile;
-//                  emits the next sort key and the next CFL maxima
-//   k_scan         exclusive scan of per-tile counts (last-block-done, one launch)
-//   k_sort_scatter counting sort: perm[start + rank] = particle, first claimer appends the tile
-//                  to the work list
+//                  emits the next CFL maxima and, when too many particles have left their tile, the next sort key
 // The scatter is dt-free (m, p = sum w (m v + m C dpos), f = -sum w (4V/h) tau dpos), so the next
 // substep's dt can be chosen on the device after the whole state is known, as the reference does
 // (src/three/simulation.js:308-310); the grid update applies dt.
@@ -79,14 +78,15 @@ __global__ void k_wait_probe(unsigned* out, long long limit) {
 
 void launch_wait_probe(cudaStream_t st, unsigned* out, long long limit) { k_wait_probe<<<1, 32, 0, st>>>(out, limit); }
 
-// 4D tiled TMA load (no multicast): box {4 channels, 6, 6, 6} of the grid velocity array.
-// The innermost coordinate is the channel index 0, so the 16-byte alignment rule holds.
-__device__ __forceinline__ void tma_load_4d(void* dst, const void* tmap, int c0, int c1, int c2, int c3,
-                                            unsigned long long* bar) {
+// 3D tiled TMA load (no multicast) of a gather window: box {4 channels x 8 nodes, 8, 8} of the grid velocity
+// array, zeros outside it. Rows of 128 bytes; with the channels as a dimension of their own the box was
+// 16-byte rows, and waiting for 512 of them cost a tile 0.9k cycles. The innermost coordinate is a multiple of four floats,
+// so the 16-byte alignment rule holds (it may be negative in a load).
+__device__ __forceinline__ void tma_load_window(void* dst, const void* tmap, int x, int y, int z, unsigned long long* bar) {
   asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, "
-      "%4, %5}], [%6];" ::"r"(smem_addr(dst)),
-      "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_addr(bar))
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, "
+      "%4}], [%5];" ::"r"(smem_addr(dst)),
+      "l"(tmap), "r"(4 * x), "r"(y), "r"(z), "r"(smem_addr(bar))
       : "memory");
 }
 
@@ -196,6 +196,8 @@ __device__ __forceinline__ void cfl_terms(const MaterialDev& mt, const float D[9
 // ---------------------------------------------------------------------------------------------
 // control
 
+constexpr unsigned kStrayShare = 32;
+
 struct ControlOp {
   int op;           // 0: reset lists for an initial sort + P2G, 1: start a step call
   int mode;
@@ -211,7 +213,7 @@ __global__ void k_control(Ctx c, ControlOp op) {
     const unsigned k = ct->step_index;
     ct->last_substep = 1u;
     if (op.op == 0) {
-      ct->work_count[k & 1] = 0;
+      ct->sort_active = ct->sort_want = ct->strays = ct->far_strays = 0u;
       ct->active_count[k & 1] = 0;
       ct->work_next = 0;
       ct->done = 0;
@@ -247,10 +249,10 @@ void launch_control_step(const Ctx& c, cudaStream_t st, int mode, double dt_req,
   k_control<<<1, 32, 0, st>>>(c, op);
 }
 
-// Substep prologue: picks dt per scene, or marks the call done.
-__global__ void __launch_bounds__(256) k_begin(Ctx c) {
+// Substep prologue, by one CTA: picks dt per scene, or marks the call done.
+__device__ __forceinline__ void begin_substep(const Ctx& c) {
   Ctrl* ct = c.ctrl;
-  __shared__ float smin[8];
+  __shared__ float smin[32];
   __shared__ int sdone;
   __shared__ float sdt;
   if (ct->done) return;
@@ -313,10 +315,15 @@ __global__ void __launch_bounds__(256) k_begin(Ctx c) {
       ct->last_substep = last ? 1u : 0u;
       const unsigned k = ct->step_index + 1;
       ct->step_index = k;
-      ct->work_count[k & 1] = 0;
       ct->active_count[k & 1] = 0;
       ct->work_next = 0;
       ct->grid_next = 0;
+      // Sort again when one particle in kStrayShare has left its tile: strays add to the buckets of phase B
+      // and to the tile's window (at 1 in 32 a full tile has about 20 more non-empty buckets than 64). A particle
+      // a whole cell out is one cell from leaving the windows, so it asks for a sort at once.
+      ct->sort_want = !ct->sort_active && (ct->far_strays != 0u || ct->strays > c.n / kStrayShare) ? 1u : 0u;
+      ct->strays = 0u;
+      ct->far_strays = 0u;
     }
     sdone = done;
     sdt = dt;
@@ -330,8 +337,6 @@ __global__ void __launch_bounds__(256) k_begin(Ctx c) {
     c.grad_max[s] = 0u;
   }
 }
-
-void launch_begin(const Ctx& c, cudaStream_t st) { k_begin<<<1, 256, 0, st>>>(c); }
 
 // ---------------------------------------------------------------------------------------------
 // counting sort by particle tile
@@ -366,8 +371,8 @@ constexpr int kScanChunk = kScanThreads * kScanPer;  // 4096 tiles per block
 // non-empty flags into rank + block_rank (a tile's place in the work list, which so comes out in
 // tile-key order). The last block to finish scans the block sums (threadfence + ticket) and sets
 // the work list's length.
-// initial: the scan of a first sort (done is clear); otherwise the scan after a scatter pass, which
-// may run beside the next substep's opening kernels and so reads the pass's own flag, not done.
+// The new list becomes the one that passes read. initial: a first sort; otherwise after a scatter pass,
+// if it wrote keys.
 __device__ __forceinline__ uint2 warp_incl_scan2(uint2 v, int lane) {
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -455,8 +460,10 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(Ctx c, int initial) {
     __syncthreads();
   }
   if (threadIdx.x == 0) {
-    const unsigned list = initial ? (c.ctrl->step_index & 1u) : c.ctrl->sort_list;
+    const unsigned list = c.ctrl->sort_list ^ 1u;
     c.ctrl->work_count[list] = carry.y;  // non-empty tiles
+    c.ctrl->sort_list = list;
+    c.ctrl->in_place = 0u;
     c.ctrl->scan_ticket = 0;
   }
 }
@@ -470,14 +477,99 @@ __device__ __forceinline__ unsigned tile_start(const Ctx& c, unsigned k) {
   return c.s.start[k] + c.s.block_off[k / kScanChunk];
 }
 
+// The same scan by one CTA, 4,096 tiles a round, after a scatter pass that wrote keys (grids of at most
+// kOpenScanTiles tiles): with most passes keeping their lists it runs once in tens of substeps, where a launch of its own
+// would cost every substep. start and rank come out global here, the block offsets zero.
+__device__ __forceinline__ void scan_tiles(const Ctx& c) {
+  __shared__ uint2 sums[kScanThreads / 32];
+  constexpr int kPer = kScanPer;
+  const int T = c.total_tiles + 1, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  uint2 carry = make_uint2(0u, 0u);
+  for (int r0 = 0; r0 < T; r0 += kScanThreads * kPer) {
+    const int base = r0 + threadIdx.x * kPer;
+    unsigned v[kPer];
+    uint2 sum = make_uint2(0u, 0u);
+#pragma unroll
+    for (int q = 0; q < kPer; q += 4) {
+      if (base + q + 4 <= c.total_tiles) {
+        const uint4 x = *reinterpret_cast<const uint4*>(c.s.count + base + q);
+        v[q] = x.x; v[q + 1] = x.y; v[q + 2] = x.z; v[q + 3] = x.w;
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[q + e] = base + q + e < c.total_tiles ? c.s.count[base + q + e] : 0u;
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+      sum.x += v[q];
+      sum.y += v[q] > 0u ? 1u : 0u;
+    }
+    const uint2 incl = warp_incl_scan2(sum, lane);
+    __syncthreads();  // sums of the round before are read
+    if (lane == 31) sums[wid] = incl;
+    __syncthreads();
+    uint2 run = make_uint2(carry.x + incl.x - sum.x, carry.y + incl.y - sum.y);
+    for (int w = 0; w < kScanThreads / 32; ++w) {
+      const uint2 x = sums[w];
+      if (w < wid) {
+        run.x += x.x;
+        run.y += x.y;
+      }
+      carry.x += x.x;
+      carry.y += x.y;
+    }
+#pragma unroll
+    for (int q = 0; q < kPer; q += 4) {
+      unsigned st[4], rk[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        st[e] = run.x;
+        rk[e] = run.y;
+        run.x += v[q + e];
+        run.y += v[q + e] > 0u ? 1u : 0u;
+      }
+      if (base + q + 4 <= T) {
+        *reinterpret_cast<uint4*>(c.s.start + base + q) = make_uint4(st[0], st[1], st[2], st[3]);
+        *reinterpret_cast<uint4*>(c.s.rank + base + q) = make_uint4(rk[0], rk[1], rk[2], rk[3]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (base + q + e < T) {
+            c.s.start[base + q + e] = st[e];
+            c.s.rank[base + q + e] = rk[e];
+          }
+      }
+    }
+  }
+  for (int b = threadIdx.x; b * kScanChunk < T; b += kScanThreads) c.s.block_off[b] = c.s.block_rank[b] = 0u;
+  if (threadIdx.x == 0) {
+    const unsigned list = c.ctrl->sort_list ^ 1u;
+    c.ctrl->work_count[list] = carry.y;  // non-empty tiles
+    c.ctrl->sort_list = list;
+    c.ctrl->in_place = 0u;
+  }
+}
+
+// Between two particle passes. scan: a scatter pass came before, and if it wrote keys its counts are
+// scanned; begin: opens the next substep.
+__global__ void __launch_bounds__(kScanThreads) k_open(Ctx c, int begin, int scan) {
+  if (scan && c.ctrl->sort_active != 0 && !(c.ctrl->status & 0x8u)) scan_tiles(c);
+  __syncthreads();
+  if (begin) begin_substep(c);
+}
+
+void launch_open(const Ctx& c, cudaStream_t st, bool begin, bool scan) {
+  if (scan && c.total_tiles > kOpenScanTiles) {
+    launch_scan(c, st, false);
+    scan = false;
+  }
+  if (begin || scan) k_open<<<1, kScanThreads, 0, st>>>(c, begin ? 1 : 0, scan ? 1 : 0);
+}
+
 // perm[start(k) + rank] = home slot; the group that claims a tile first writes its work item.
-// After a scatter pass the sort may run beside the next substep's k_begin and grid update, so it
-// takes its list and its go-ahead from the fields that pass wrote (sort_list, sort_active), which
-// k_begin does not touch.
-__global__ void __launch_bounds__(256) k_sort_scatter(Ctx c, int initial) {
-  if (!initial && c.ctrl->sort_active == 0) return;
-  if (c.ctrl->status & 0x8u) return;  // a bounded wait gave up this substep
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+// block: index of the 256-particle block.
+__device__ __forceinline__ void sort_scatter(const Ctx& c, long long block) {
+  const long long i = block * 256 + threadIdx.x;
   const unsigned key = i < c.n ? c.p.key[i] : 0xffffffffu;
   const unsigned mask = __match_any_sync(0xffffffffu, key);
   if (key == 0xffffffffu) return;
@@ -497,16 +589,22 @@ __global__ void __launch_bounds__(256) k_sort_scatter(Ctx c, int initial) {
   }
   c.p.perm[s0 + old - 1 - below] = static_cast<unsigned>(i);
   if (lane == leader && old == cnt) {  // the tile's first group writes its work item at the tile's rank
-    const unsigned list = initial ? (c.ctrl->step_index & 1u) : c.ctrl->sort_list;
+    const unsigned list = c.ctrl->sort_list;
     const unsigned idx = c.s.rank[key] + c.s.block_rank[key / kScanChunk];
     const int s = c.nscenes == 1 ? 0 : find_scene_by_tile(c.scenes, c.nscenes, static_cast<int>(key));
     if (idx < static_cast<unsigned>(c.total_tiles)) c.s.work[list][idx] = make_uint4(key, s0, cnt, static_cast<unsigned>(s));
   }
 }
 
-void launch_sort_scatter(const Ctx& c, cudaStream_t st, bool initial) {
+// The first sort of a state.
+__global__ void __launch_bounds__(256) k_sort_scatter(Ctx c) {
+  if (c.ctrl->status & 0x8u) return;  // a bounded wait gave up
+  sort_scatter(c, blockIdx.x);
+}
+
+void launch_sort_scatter(const Ctx& c, cudaStream_t st) {
   const long long blocks = (c.n + 255) / 256;
-  if (blocks > 0) k_sort_scatter<<<static_cast<unsigned>(blocks), 256, 0, st>>>(c, initial ? 1 : 0);
+  if (blocks > 0) k_sort_scatter<<<static_cast<unsigned>(blocks), 256, 0, st>>>(c);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -527,9 +625,9 @@ void launch_sort_scatter(const Ctx& c, cudaStream_t st, bool initial) {
 
 // Particles per scatter round. A full tile holds 512 (64 cells x 8), but a block that drifts by a
 // fraction of a cell leaves a third of its tiles a few particles over 512 (up to ~530); at a cap of
-// 512 those took a second round (every phase and barrier again for a handful of particles). 608 is
+// 512 those took a second round (every phase and barrier again for a handful of particles). 592 is
 // what two CTAs per SM leave beside the window copies.
-constexpr int kCap = 608;
+constexpr int kCap = 592;
 constexpr int kWinCopyNodes = 6 * kWinS * kWinS;  // nodes of one window copy: six bucket layers
 constexpr int kPf = 2;         // perm entries of the next tile's first round held per thread (shared memory)
 // Payload of one particle: six float4 rows laid out for the paired FMAs of phase B:
@@ -544,6 +642,7 @@ constexpr int kBuckets = 216;  // 6^3 possible stencil bases in the scatter wind
 __device__ __forceinline__ int pay_slot(int j) { return j ^ ((j >> 3) & 7); }
 static_assert(kCap % 8 == 0, "pay_slot permutes within blocks of eight");
 constexpr unsigned kMetaInvalid = 0x80000000u;
+constexpr unsigned kFlagFar = 0x80000000u;  // beside the status flags: a stray a whole cell out of its tile
 
 enum Pass : int { kPassP2G = 0, kPassG2P2G = 1, kPassG2P = 2 };
 
@@ -561,7 +660,7 @@ struct TileCtx {
 };
 
 struct __align__(128) PartSmem {
-  float4 vwin[2][kWinG * kWinG * kWinG];  // double-buffered TMA destinations (3456 B each)
+  float4 vwin[kWinG * kWinG * kWinG];     // TMA destination (8 KiB): free again once a tile's last phase A is over
   float4 win[3][2][kWinCopyNodes];        // 36 KiB scatter window (see win_node)
   float4 pay[kPayRows * kCap];            // 57 KiB payloads, structure of float4 arrays (swizzled slots)
   unsigned meta[kCap];                    // bucket | rank << 8 (or kMetaInvalid)
@@ -571,16 +670,18 @@ struct __align__(128) PartSmem {
   unsigned short blist[kBuckets];
   int nbuckets;
   int wsum[kBlock / 32], wnz[kBlock / 32];  // per-warp bucket totals of the block-wide scan
-  unsigned long long mbar[2];
+  unsigned long long mbar;
   uint4 item[2];
   int abort_flag;
-  unsigned red[3];   // the tile's CFL maxima (float bits) and status flags
+  unsigned red[4];   // the tile's CFL maxima (float bits), status flags (and kFlagFar), strays
   unsigned gate[2];  // learned mode: returns the gate accepted / sent to the bisection
   // State the CTA carries from tile to tile sits here rather than in registers: at 128 registers a
   // thread, every register held across the tiles is one fewer for phase A, and moving these (with
   // the heat sum, which was a per-thread double) cut the pass by 7%.
-  unsigned tma_phase[2];       // mbarrier phases of the two window buffers (thread 0)
+  unsigned tma_phase;          // mbarrier phase of the window buffer (thread 0)
   double work_sum;             // heat from plastic work of the CTA's particles
+  const uint4* work;           // the list this pass reads, its length, and whether perm is the identity
+  unsigned work_count, in_place;
   unsigned pfs[kPf * kBlock];  // perm entries j of the next tile's first round, j < kPf x kBlock
 
   TileCtx tc[2];               // by item buffer
@@ -958,11 +1059,19 @@ __device__ __noinline__ Gather12 gather_global(const float4* base, int sy, long 
   return g;
 }
 
+// A stray (window bases 1..4 are the tile's, 0 and 5 one cell out) within a quarter cell of leaving the
+// windows.
+__device__ __forceinline__ bool near_window_end(int l0, float t0, int l1, float t1, int l2, float t2) {
+  return (l0 == 0 && t0 < 0.75f) || (l0 == 5 && t0 > 1.25f) || (l1 == 0 && t1 < 0.75f) || (l1 == 5 && t1 > 1.25f) ||
+         (l2 == 0 && t2 < 0.75f) || (l2 == 5 && t2 > 1.25f);
+}
+
 // Phase A of one particle (home slot `home`, payload row j): G2P from the staged window, F update,
 // fixed-point advection and the constitutive update / return map (src/three/mpm.js:107-131), or,
 // for the P2G pass and pinned particles, the stress of the stored state; then the scatter payload
 // bucketed by its new stencil base in the shared window (pay, meta, hist), and the CFL terms.
-// Writes the particle's new state and returns its next sort key (all ones when not needed).
+// Writes the particle's new state and returns its next sort key (all ones unless want is set); stray: its new base
+// lies outside the tile.
 // NEWTON (the Newton-gated return mode): a Johnson-Cook trial stress above the initial flow stress
 // takes the gated refinement from u0 = 1 - flow(ep, 0, T) / q instead of the bisection, which stays
 // the fallback; gate[0] / gate[1] count the returns accepted / sent to the bisection.
@@ -972,7 +1081,7 @@ __device__ __forceinline__ unsigned particle_phase_a(const Ctx& c, const SceneDe
                                                      unsigned home, unsigned j, float dt, int nxt, float4* pay,
                                                      unsigned* meta, int* hist, float& wave_acc, float& grad_acc,
                                                      unsigned& flags_acc, double& work_acc, bool store_vc,
-                                                     unsigned* gate = nullptr) {
+                                                     bool want, bool& stray, unsigned* gate = nullptr) {
   static_assert(!NEWTON || (!HEAT && !AUX && PASS != kPassP2G), "Newton-gated returns: J2-type laws, gather passes");
   constexpr bool SCATTER = PASS != kPassG2P;
   constexpr bool GATHER = PASS != kPassP2G;
@@ -999,11 +1108,10 @@ __device__ __forceinline__ unsigned particle_phase_a(const Ctx& c, const SceneDe
       stencil_axis(q[a], tc.dims[a], b[a], t[a]);
       bspline_weights(t[a], w[a]);
     }
-    const int l0 = b[0] - tc.tile[0] * kTile, l1 = b[1] - tc.tile[1] * kTile, l2 = b[2] - tc.tile[2] * kTile;
-    // the sort key places the stencil inside the staged window; if it ever does not, the
-    // particle reads the grid from global memory instead (and the step reports it)
+    // the window reaches one cell out of the tile on each side, so a particle may leave the tile it is listed
+    // in; one that is further out reads the grid from global memory
+    const int l0 = b[0] - (tc.tile[0] * kTile - 1), l1 = b[1] - (tc.tile[1] * kTile - 1), l2 = b[2] - (tc.tile[2] * kTile - 1);
     const bool in_g = l0 >= 0 && l0 <= kWinG - 3 && l1 >= 0 && l1 <= kWinG - 3 && l2 >= 0 && l2 <= kWinG - 3;
-    if (!in_g) flags |= 0x20u;
     // G2P (src/three/mpm.js:107-118): v = sum w v_i, C = sum w v_i (i - t)^T 4/h
     float acc12[12];
     if (in_g) {
@@ -1128,8 +1236,10 @@ __device__ __forceinline__ unsigned particle_phase_a(const Ctx& c, const SceneDe
     float t[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) stencil_axis(q[a], tc.dims[a], nb[a], t[a]);
-    key = tile_key(sc, nb);
-    if (PASS == kPassG2P2G) c.p.key[home] = key;
+    if (PASS == kPassG2P2G && want) {
+      key = tile_key(sc, nb);
+      c.p.key[home] = key;
+    }
     const float mv[3] = {m * v[0], m * v[1], m * v[2]};
     const float mH = m * tc.H;
     float mC[9];
@@ -1140,6 +1250,10 @@ __device__ __forceinline__ unsigned particle_phase_a(const Ctx& c, const SceneDe
     const int l0 = nb[0] - (tc.tile[0] * kTile - 1), l1 = nb[1] - (tc.tile[1] * kTile - 1),
               l2 = nb[2] - (tc.tile[2] * kTile - 1);
     const bool in_w = l0 >= 0 && l0 <= kWinS - 3 && l1 >= 0 && l1 <= kWinS - 3 && l2 >= 0 && l2 <= kWinS - 3;
+    if (PASS == kPassG2P2G && in_w) {
+      stray = (((l0 - 1) | (l1 - 1) | (l2 - 1)) & ~3) != 0;
+      if (stray && near_window_end(l0, t[0], l1, t[1], l2, t[2])) flags |= kFlagFar;
+    }
     if (in_w && !pinned) {
       const int bucket = (l2 * 6 + l1) * 6 + l0;
       // one shared atomic per bucket among the warp's converged lanes (particles of one cell share
@@ -1157,7 +1271,12 @@ __device__ __forceinline__ unsigned particle_phase_a(const Ctx& c, const SceneDe
       P[5 * kCap] = make_float4(mC[6], s6[0], s6[1], s6[5]);
     } else {
       meta[j] = kMetaInvalid;
-      if (!in_w) flags |= 0x10u;
+      if (!in_w) {
+        stray = true;
+        flags |= kFlagFar;
+        const float cells = dt * tc.invH;  // more than a cell in this substep
+        if (fabsf(cells * v[0]) > 1.f || fabsf(cells * v[1]) > 1.f || fabsf(cells * v[2]) > 1.f) flags |= 0x10u;
+      }
       // copies scoped to this rare branch: the arrays passed to the out-of-line scatter would
       // otherwise live in local memory on every particle's path (3% of the fused pass)
       int nb_g[3];
@@ -1224,7 +1343,8 @@ __device__ __forceinline__ unsigned particle_phase_a_learned(const Ctx& c, const
                                                              const float4* vwin, bool live, unsigned home, unsigned j,
                                                              float dt, int nxt, float4* pay, unsigned* meta, int* hist,
                                                              float& wave_acc, float& grad_acc, unsigned& flags_acc,
-                                                             double& work_acc, bool store_vc, unsigned* gate) {
+                                                             double& work_acc, bool store_vc, bool want, bool& stray,
+                                                             unsigned* gate) {
   constexpr bool SCATTER = PASS != kPassG2P;
   static_assert(PASS != kPassP2G, "the learned mode changes only returns");
   unsigned key = 0xffffffffu;
@@ -1251,9 +1371,8 @@ __device__ __forceinline__ unsigned particle_phase_a_learned(const Ctx& c, const
       stencil_axis(q[a], tc.dims[a], b[a], t[a]);
       bspline_weights(t[a], w[a]);
     }
-    const int l0 = b[0] - tc.tile[0] * kTile, l1 = b[1] - tc.tile[1] * kTile, l2 = b[2] - tc.tile[2] * kTile;
+    const int l0 = b[0] - (tc.tile[0] * kTile - 1), l1 = b[1] - (tc.tile[1] * kTile - 1), l2 = b[2] - (tc.tile[2] * kTile - 1);
     const bool in_g = l0 >= 0 && l0 <= kWinG - 3 && l1 >= 0 && l1 <= kWinG - 3 && l2 >= 0 && l2 <= kWinG - 3;
-    if (!in_g) flags |= 0x20u;
     float acc12[12];
     if (in_g) {
       const float4* win = &vwin[(l2 * kWinG + l1) * kWinG + l0];
@@ -1351,8 +1470,10 @@ __device__ __forceinline__ unsigned particle_phase_a_learned(const Ctx& c, const
     float t[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) stencil_axis(q[a], tc.dims[a], nb[a], t[a]);
-    key = tile_key(sc, nb);
-    if (PASS == kPassG2P2G) c.p.key[home] = key;
+    if (PASS == kPassG2P2G && want) {
+      key = tile_key(sc, nb);
+      c.p.key[home] = key;
+    }
     const float mv[3] = {m * v[0], m * v[1], m * v[2]};
     const float mH = m * tc.H;
     float mC[9];
@@ -1363,6 +1484,10 @@ __device__ __forceinline__ unsigned particle_phase_a_learned(const Ctx& c, const
     const int l0 = nb[0] - (tc.tile[0] * kTile - 1), l1 = nb[1] - (tc.tile[1] * kTile - 1),
               l2 = nb[2] - (tc.tile[2] * kTile - 1);
     const bool in_w = l0 >= 0 && l0 <= kWinS - 3 && l1 >= 0 && l1 <= kWinS - 3 && l2 >= 0 && l2 <= kWinS - 3;
+    if (PASS == kPassG2P2G && in_w) {
+      stray = (((l0 - 1) | (l1 - 1) | (l2 - 1)) & ~3) != 0;
+      if (stray && near_window_end(l0, t[0], l1, t[1], l2, t[2])) flags |= kFlagFar;
+    }
     if (in_w && !pinned) {
       const int bucket = (l2 * 6 + l1) * 6 + l0;
       // one shared integer atomic per particle: grouping the warp's lanes by bucket first
@@ -1378,7 +1503,12 @@ __device__ __forceinline__ unsigned particle_phase_a_learned(const Ctx& c, const
       P[5 * kCap] = make_float4(mC[6], s6[0], s6[1], s6[5]);
     } else {
       meta[j] = kMetaInvalid;
-      if (!in_w) flags |= 0x10u;
+      if (!in_w) {
+        stray = true;
+        flags |= kFlagFar;
+        const float cells = dt * tc.invH;  // more than a cell in this substep
+        if (fabsf(cells * v[0]) > 1.f || fabsf(cells * v[1]) > 1.f || fabsf(cells * v[2]) > 1.f) flags |= 0x10u;
+      }
       // copies scoped to this rare branch: the arrays passed to the out-of-line scatter would
       // otherwise live in local memory on every particle's path
       int nb_g[3];
@@ -1405,17 +1535,25 @@ __device__ __forceinline__ unsigned particle_phase_a_learned(const Ctx& c, const
   return key;
 }
 
-// L2 prefetch of the particle state a claimed tile will read. Between physical re-sorts a tile's
-// particles keep the contiguous home range the last re-sort gave them (apart from the few that
-// changed tiles since), and the tile's perm lists them in about that order; one perm entry from the
+// L2 prefetch of the particle state a claimed tile will read. After a permutation the tile's particles are
+// one range (in_place). Between it and the next one they keep that range apart from the few that
+// changed tiles, and the tile's perm lists them in about that order; one perm entry from the
 // middle places the range, and one bulk prefetch per state array covers it with a margin. Only a
 // hint: the range is clipped to the live particles and a wrong guess costs bandwidth, not results.
 template <bool AUX>
-__device__ __forceinline__ void prefetch_tile_state(const Ctx& c, uint4 it) {
+__device__ __forceinline__ void prefetch_tile_state(const Ctx& c, uint4 it, bool in_place) {
   const long long cnt = it.z;
   if (cnt == 0) return;
-  const long long mid = c.p.perm[it.y + it.z / 2];
-  const long long lo = max(0ll, mid - (3 * cnt) / 4 - 32), hi = min(static_cast<long long>(c.n), mid + (3 * cnt) / 4 + 32);
+  long long lo = it.y, hi = it.y + cnt;
+  if (!in_place) {
+    // the list itself: it was written some passes ago and may have left L2
+    const unsigned long long a = reinterpret_cast<unsigned long long>(c.p.perm + lo) & ~15ull;
+    const unsigned long long b = (reinterpret_cast<unsigned long long>(c.p.perm + hi) + 15) & ~15ull;
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"(static_cast<unsigned>(b - a)) : "memory");
+    const long long mid = c.p.perm[it.y + it.z / 2];
+    lo = max(0ll, mid - (3 * cnt) / 4 - 32);
+    hi = min(static_cast<long long>(c.n), mid + (3 * cnt) / 4 + 32);
+  }
   if (hi <= lo) return;
   auto pf = [&](const void* base, int esize) {
     const unsigned long long a = (reinterpret_cast<unsigned long long>(base) + lo * esize) & ~15ull;
@@ -1448,25 +1586,24 @@ __global__ void __launch_bounds__(kBlock, 2) k_particles(const __grid_constant__
   constexpr bool GATHER = PASS != kPassP2G;
   constexpr unsigned kNone = 0xffffffffu;
   Ctrl* ct = c.ctrl;
-  if (PASS == kPassG2P2G && blockIdx.x == 0 && threadIdx.x == 0) {  // for the sort that follows
-    ct->sort_list = ct->step_index & 1u;
-    ct->sort_active = ct->done ? 0u : 1u;
-  }
+  // Most passes keep the tile lists of an earlier sort: a particle moves a thousandth of a cell per substep
+  // in a stiff metal, and the windows reach one cell out of the tile. A pass that does write keys is
+  // followed by the scan and the sort.
+  const bool want = PASS == kPassG2P2G && (ct->sort_want != 0u || c.force_sort != 0);
+  if (PASS == kPassG2P2G && blockIdx.x == 0 && threadIdx.x == 0) ct->sort_active = want && !ct->done ? 1u : 0u;
   if (PASS != kPassP2G && ct->done) return;
   const unsigned k = ct->step_index;
   const bool store_vc = ct->last_substep != 0u;
-  // lists: the P2G pass reads the list its sort just wrote (k & 1) and scatters into acc[k & 1];
-  // a substep (after k_begin advanced k) reads list (k - 1) & 1 and scatters into acc[k & 1]
-  const int lst = PASS == kPassP2G ? (k & 1) : ((k - 1) & 1);
-  const int nxt = k & 1;
+  const int nxt = k & 1;  // the pass scatters into acc[k & 1] (k_begin advanced k before a substep)
   const bool use_tma = GATHER && c.use_tma;
   const bool single = c.single_material != 0 || c.scene_material != 0;
 
   // One thread claims a work item for buffer `buf`: item, tile constants, the velocity window's TMA
   // and the L2 prefetch of the tile's particles.
-  auto claim = [&](int buf) {
-    const unsigned idx = atomicAdd(&ct->work_next, 1u);
-    const uint4 nx = idx < ct->work_count[lst] ? c.s.work[lst][idx] : make_uint4(kNone, 0, 0, 0);
+  auto claim = [&](int buf, bool first) {
+    // each CTA's first item is its own index, the rest are claimed
+    const unsigned idx = first ? blockIdx.x : gridDim.x + atomicAdd(&ct->work_next, 1u);
+    const uint4 nx = idx < sm.work_count ? sm.work[idx] : make_uint4(kNone, 0, 0, 0);
     sm.item[buf] = nx;
     if (nx.x == kNone) return;
     const SceneDev& sc = c.scenes[nx.w];
@@ -1475,9 +1612,9 @@ __global__ void __launch_bounds__(kBlock, 2) k_particles(const __grid_constant__
     const int tx = lt % sc.tiles[0], ty = (lt / sc.tiles[0]) % sc.tiles[1], tz = lt / (sc.tiles[0] * sc.tiles[1]);
     if (use_tma && !sm.abort_flag) {
       fence_proxy_async_smem();
-      mbar_arrive_expect_tx(&sm.mbar[buf], sizeof(sm.vwin[0]));
-      tma_load_4d(sm.vwin[buf], static_cast<const char*>(c.tmaps) + 128 * nx.w, 0, tx * kTile, ty * kTile, tz * kTile,
-                  &sm.mbar[buf]);
+      mbar_arrive_expect_tx(&sm.mbar, sizeof(sm.vwin));
+      tma_load_window(sm.vwin, static_cast<const char*>(c.tmaps) + 128 * nx.w, tx * kTile - 1, ty * kTile - 1, tz * kTile - 1,
+                      &sm.mbar);
     }
     tl.tile[0] = tx;
     tl.tile[1] = ty;
@@ -1495,7 +1632,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_particles(const __grid_constant__
     tl.clamp = sc.clamp;
     tl.mat = sc.mat_base;
     tl.dt = GATHER ? c.dt_scene[nx.w] : 0.f;
-    prefetch_tile_state<AUX>(c, nx);
+    prefetch_tile_state<AUX>(c, nx, sm.in_place != 0u);
   };
   // Every thread of the CTA, between two tiles: what the next tile (buffer buf, already claimed) needs
   // before phase A, in the shadow of the previous tile's flush.
@@ -1505,7 +1642,10 @@ __global__ void __launch_bounds__(kBlock, 2) k_particles(const __grid_constant__
 #pragma unroll
     for (int q = 0; q < kPf; ++q) {
       const unsigned j = q * kBlock + threadIdx.x;
-      pf[q] = nx.x != kNone && j < nx.z ? c.p.perm[nx.y + j] : 0u;
+      pf[q] = nx.y + j;
+      // volatile: issued here, before the flush, not sunk to its use behind it
+      if (!sm.in_place && nx.x != kNone && j < nx.z)
+        asm volatile("ld.global.u32 %0, [%1];" : "=r"(pf[q]) : "l"(c.p.perm + nx.y + j) : "memory");
     }
   };
   auto finish_next = [&](int buf, int mat_now) {
@@ -1523,19 +1663,21 @@ __global__ void __launch_bounds__(kBlock, 2) k_particles(const __grid_constant__
     if (GATHER && !use_tma) {
       const TileCtx& tl = sm.tc[buf];
       for (int i = threadIdx.x; i < kWinG * kWinG * kWinG; i += kBlock) {
-        const int x = tl.tile[0] * kTile + i % kWinG, y = tl.tile[1] * kTile + (i / kWinG) % kWinG,
-                  z = tl.tile[2] * kTile + i / (kWinG * kWinG);
-        sm.vwin[buf][i] = c.g.vel[tl.node_base + ((long long)z * tl.gdim[1] + y) * tl.gdim[0] + x];
+        const int x = tl.tile[0] * kTile - 1 + i % kWinG, y = tl.tile[1] * kTile - 1 + (i / kWinG) % kWinG,
+                  z = tl.tile[2] * kTile - 1 + i / (kWinG * kWinG);
+        sm.vwin[i] = x >= 0 && y >= 0 && z >= 0 && x < tl.gdim[0] && y < tl.gdim[1] && z < tl.gdim[2]
+                         ? c.g.vel[tl.node_base + ((long long)z * tl.gdim[1] + y) * tl.gdim[0] + x]
+                         : make_float4(0.f, 0.f, 0.f, 0.f);
       }
     }
     if (use_tma && threadIdx.x == 0) {
-      const unsigned ph = sm.tma_phase[buf];
-      if (!mbar_wait_bounded(&sm.mbar[buf], ph)) {
+      const unsigned ph = sm.tma_phase;
+      if (!mbar_wait_bounded(&sm.mbar, ph)) {
         atomicOr(&ct->status, 0x8u);
-        mbar_wait_bounded(&sm.mbar[buf], ph);  // a second bounded chance for the copy in flight
+        mbar_wait_bounded(&sm.mbar, ph);  // a second bounded chance for the copy in flight
         sm.abort_flag = 1;
       }
-      sm.tma_phase[buf] ^= 1u;
+      sm.tma_phase ^= 1u;
     }
   };
 
@@ -1544,15 +1686,18 @@ __global__ void __launch_bounds__(kBlock, 2) k_particles(const __grid_constant__
     for (int i = threadIdx.x; i < kBuckets; i += kBlock) sm.hist[i] = 0;
   }
   if (threadIdx.x == 0) {
-    mbar_init(&sm.mbar[0], 1);
-    mbar_init(&sm.mbar[1], 1);
+    mbar_init(&sm.mbar, 1);
     fence_barrier_init();
     sm.abort_flag = 0;
     sm.gate[0] = sm.gate[1] = 0u;
-    sm.tma_phase[0] = sm.tma_phase[1] = 0u;
+    sm.tma_phase = 0u;
+    const unsigned lst = ct->sort_list;
+    sm.in_place = ct->in_place;
+    sm.work_count = ct->work_count[lst];
+    sm.work = c.s.work[lst];
     sm.work_sum = 0.0;
-    sm.red[0] = sm.red[1] = sm.red[2] = 0u;
-    claim(0);
+    sm.red[0] = sm.red[1] = sm.red[2] = sm.red[3] = 0u;
+    claim(0, true);
   }
   __syncthreads();
   load_perm(0);
@@ -1560,7 +1705,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_particles(const __grid_constant__
   __syncthreads();
   for (int cb = 0;; cb ^= 1) {
     if (sm.item[cb].x == kNone) break;
-    if (sm.abort_flag) return;
+    if (sm.abort_flag) break;
     const TileCtx& tc = sm.tc[cb];
     for (unsigned r0 = 0; r0 < sm.item[cb].z; r0 += kCap) {
       const unsigned nround = min(static_cast<unsigned>(kCap), sm.item[cb].z - r0);
@@ -1573,28 +1718,32 @@ __global__ void __launch_bounds__(kBlock, 2) k_particles(const __grid_constant__
         unsigned key = kNone;
         float wave = 0.f, grad = 0.f;
         unsigned flags = 0;
+        bool stray = false;
         const SceneDev& sc = c.scenes[sm.item[cb].w];
         if constexpr (JC == 1) {
           // every lane of a warp with a live particle takes part in its network evaluation
           const unsigned home = !live ? c.p.perm[sm.item[cb].y + r0]
                                       : (r0 == 0 && jj < kPf * kBlock) ? sm.pfs[j] : c.p.perm[sm.item[cb].y + r0 + j];
-          key = particle_phase_a_learned<PASS>(c, sc, tc, sm.mt, single, sm.vwin[cb], live, home, j, tc.dt, nxt, sm.pay,
-                                               sm.meta, sm.hist, wave, grad, flags, sm.work_sum, store_vc, sm.gate);
+          key = particle_phase_a_learned<PASS>(c, sc, tc, sm.mt, single, sm.vwin, live, home, j, tc.dt, nxt, sm.pay,
+                                               sm.meta, sm.hist, wave, grad, flags, sm.work_sum, store_vc, want, stray,
+                                               sm.gate);
         } else if (live) {
           const unsigned home = (r0 == 0 && jj < kPf * kBlock) ? sm.pfs[j] : c.p.perm[sm.item[cb].y + r0 + j];
-          key = particle_phase_a<PASS, HEAT, AUX, JC == 2>(c, sc, tc, sm.mt, single, sm.vwin[cb], home, j, tc.dt, nxt,
-                                                           sm.pay, sm.meta, sm.hist, wave, grad, flags, sm.work_sum,
-                                                           store_vc, sm.gate);
+          key = particle_phase_a<PASS, HEAT, AUX, JC == 2>(c, sc, tc, sm.mt, single, sm.vwin, home, j, tc.dt, nxt, sm.pay,
+                                                           sm.meta, sm.hist, wave, grad, flags, sm.work_sum, store_vc,
+                                                           want, stray, sm.gate);
         }
-        if (PASS == kPassG2P2G) count_key(c, key);
-        // CFL maxima and status flags of the tile
+        if (want) count_key(c, key);
+        // CFL maxima, status flags and strays of the tile
         const unsigned wb = __reduce_max_sync(0xffffffffu, fbits(wave));
         const unsigned gb = __reduce_max_sync(0xffffffffu, fbits(grad));
         const unsigned fl = __reduce_or_sync(0xffffffffu, flags);
+        const unsigned out = __ballot_sync(0xffffffffu, stray);
         if ((threadIdx.x & 31) == 0) {
           atomicMax(&sm.red[0], wb);
           atomicMax(&sm.red[1], gb);
           if (fl) atomicOr(&sm.red[2], fl);
+          if (out) atomicAdd(&sm.red[3], __popc(out));
         }
       }
       // the last thread claims the next tile (a full tile has about 3 x 64 phase-B tasks, so its warp
@@ -1608,24 +1757,29 @@ __global__ void __launch_bounds__(kBlock, 2) k_particles(const __grid_constant__
           if (!(mm & kMetaInvalid)) sm.sidx[sm.bstart[mm & 0xffu] + (mm >> 8)] = static_cast<unsigned short>(j);
         }
         __syncthreads();
+        // the window buffer is free after the last round's phase A
+        if (r0 + kCap >= sm.item[cb].z && threadIdx.x == kBlock - 1) claim(cb ^ 1, false);
         if (r0 == 0) {
-          if (threadIdx.x == kBlock - 1) claim(cb ^ 1);
           const int lane27 = static_cast<int>(threadIdx.x) - (kBlock - 64);
           if (lane27 >= 0 && lane27 < 27) mark_window(c, c.scenes[sm.item[cb].w], nxt, tc.tile, lane27);
         }
         phase_b<HEAT>(sm, sm.nbuckets);  // ends at a barrier
-      } else if (r0 == 0) {
-        if (threadIdx.x == kBlock - 1) claim(cb ^ 1);
       }
     }
-    if (!SCATTER) __syncthreads();
+    if (!SCATTER) {
+      __syncthreads();
+      if (threadIdx.x == kBlock - 1) claim(cb ^ 1, false);
+      __syncthreads();
+    }
     load_perm(cb ^ 1);
     if (threadIdx.x == 32) {
       const unsigned scene = sm.item[cb].w;
       atomicMax(&c.wave_max[scene], sm.red[0]);
       atomicMax(&c.grad_max[scene], sm.red[1]);
-      if (sm.red[2]) atomicOr(&ct->status, sm.red[2]);
-      sm.red[0] = sm.red[1] = sm.red[2] = 0u;
+      if (sm.red[2] & ~kFlagFar) atomicOr(&ct->status, sm.red[2] & ~kFlagFar);
+      if (sm.red[2] & kFlagFar) atomicOr(&ct->far_strays, 1u);
+      if (sm.red[3]) atomicAdd(&ct->strays, sm.red[3]);
+      sm.red[0] = sm.red[1] = sm.red[2] = sm.red[3] = 0u;
     }
     if (SCATTER) flush_window(c, c.scenes[sm.item[cb].w], sm, nxt, tc.tile);
     finish_next(cb ^ 1, tc.mat);
@@ -1728,14 +1882,11 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_particles_ws(const __grid_con
   WsSmem& sm = *reinterpret_cast<WsSmem*>(smem_raw);
   constexpr bool GATHER = PASS != kPassP2G;
   Ctrl* ct = c.ctrl;
-  if (PASS == kPassG2P2G && blockIdx.x == 0 && threadIdx.x == 0) {  // for the sort that follows
-    ct->sort_list = ct->step_index & 1u;
-    ct->sort_active = ct->done ? 0u : 1u;
-  }
+  if (PASS == kPassG2P2G && blockIdx.x == 0 && threadIdx.x == 0) ct->sort_active = ct->done ? 0u : 1u;  // sorts every pass
   if (PASS != kPassP2G && ct->done) return;
   const unsigned k = ct->step_index;
   const bool store_vc = ct->last_substep != 0u;
-  const int lst = PASS == kPassP2G ? (k & 1) : ((k - 1) & 1);
+  const int lst = ct->sort_list;
   const int nxt = k & 1;
   const bool use_tma = GATHER && c.use_tma;
   for (int i = threadIdx.x; i < kChannels * kWinSNodes; i += kWsThreads) sm.acc[i] = 0.f;
@@ -1744,8 +1895,8 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_particles_ws(const __grid_con
     const int lt = static_cast<int>(it.x) - sn.tile_base;
     fence_proxy_async_smem();
     mbar_arrive_expect_tx(&sm.tma_bar[buf], sizeof(sm.vwin[0]));
-    tma_load_4d(sm.vwin[buf], static_cast<const char*>(c.tmaps) + 128 * it.w, 0, (lt % sn.tiles[0]) * kTile,
-                ((lt / sn.tiles[0]) % sn.tiles[1]) * kTile, (lt / (sn.tiles[0] * sn.tiles[1])) * kTile,
+    tma_load_window(sm.vwin[buf], static_cast<const char*>(c.tmaps) + 128 * it.w, (lt % sn.tiles[0]) * kTile - 1,
+                ((lt / sn.tiles[0]) % sn.tiles[1]) * kTile - 1, (lt / (sn.tiles[0] * sn.tiles[1])) * kTile - 1,
                 &sm.tma_bar[buf]);
   };
   if (threadIdx.x == 0) {
@@ -1821,9 +1972,11 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_particles_ws(const __grid_con
       if (GATHER && !use_tma) {
         const TileCtx& tl = sm.tc;
         for (int i = tid; i < kWinG * kWinG * kWinG; i += kWsGroup) {
-          const int x = tl.tile[0] * kTile + i % kWinG, y = tl.tile[1] * kTile + (i / kWinG) % kWinG,
-                    z = tl.tile[2] * kTile + i / (kWinG * kWinG);
-          sm.vwin[cb][i] = c.g.vel[tl.node_base + ((long long)z * tl.gdim[1] + y) * tl.gdim[0] + x];
+          const int x = tl.tile[0] * kTile - 1 + i % kWinG, y = tl.tile[1] * kTile - 1 + (i / kWinG) % kWinG,
+                    z = tl.tile[2] * kTile - 1 + i / (kWinG * kWinG);
+          sm.vwin[cb][i] = x >= 0 && y >= 0 && z >= 0 && x < tl.gdim[0] && y < tl.gdim[1] && z < tl.gdim[2]
+                               ? c.g.vel[tl.node_base + ((long long)z * tl.gdim[1] + y) * tl.gdim[0] + x]
+                               : make_float4(0.f, 0.f, 0.f, 0.f);
         }
         group_sync(1);
       }
@@ -1851,10 +2004,12 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_particles_ws(const __grid_con
         for (unsigned jj = 0; jj < nround; jj += kWsGroup) {
           const unsigned j = jj + tid;
           unsigned key = 0xffffffffu;
+          bool stray = false;
           if (j < nround) {
             const unsigned home = c.p.perm[it.y + r0 + j];
             key = particle_phase_a<PASS, HEAT, AUX>(c, sc, tc, sm.mt, single, sm.vwin[cb], home, j, dt, nxt, sm.pay[s],
-                                         sm.meta[s], sm.hist[s], wave_acc, grad_acc, flags_acc, sm.work_sum, store_vc);
+                                         sm.meta[s], sm.hist[s], wave_acc, grad_acc, flags_acc, sm.work_sum, store_vc, true,
+                                         stray);
           }
           if (PASS == kPassG2P2G) count_key(c, key);
         }
@@ -1876,7 +2031,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_particles_ws(const __grid_con
         s ^= 1;
       }
       if (stop) break;
-      group_reduce_item(c, scene, wave_acc, grad_acc, flags_acc, sm.red, tid);
+      group_reduce_item(c, scene, wave_acc, grad_acc, flags_acc & ~kFlagFar, sm.red, tid);
       cb ^= 1;
     }
     // sentinel stage: the consumer leaves after it. A group that stopped early first lets its own
@@ -2019,14 +2174,14 @@ int p2g_blocks_per_sm() { return blocks_per_sm<kPassP2G>(); }
 
 
 // Grid update over the active node tiles (src/three/mpm.js:89-102 with gravity on the grid).
-__global__ void __launch_bounds__(256) k_grid_update(Ctx c) {
+__device__ __forceinline__ void grid_update(const Ctx& c, unsigned block, unsigned blocks) {
   Ctrl* ct = c.ctrl;
   if (ct->done) return;
   const unsigned k = ct->step_index;
   const int cur = (k - 1) & 1;
   const unsigned count = ct->active_count[cur];
   const int sub = threadIdx.x >> 6, lid = threadIdx.x & 63;
-  for (unsigned ti = blockIdx.x * 4 + sub; ti < count; ti += gridDim.x * 4) {
+  for (unsigned ti = block * 4 + sub; ti < count; ti += blocks * 4) {
     const unsigned tile = c.g.active[cur][ti];
     const int s = c.nscenes == 1 ? 0 : find_scene_by_node_tile(c.scenes, c.nscenes, static_cast<int>(tile));
     const SceneDev& sc = c.scenes[s];
@@ -2062,6 +2217,18 @@ __global__ void __launch_bounds__(256) k_grid_update(Ctx c) {
     }
     if (lid == 0) c.g.tile_flag[tile] = 0u;
   }
+}
+
+// One launch between two particle passes: the first grid_blocks CTAs update the grid, the rest sort the
+// last pass's keys, if it wrote any. The two touch different data (the sort: keys, counts, perm and the newest
+// work list).
+__global__ void __launch_bounds__(256) k_grid_sort(Ctx c, unsigned grid_blocks) {
+  if (blockIdx.x < grid_blocks) {
+    grid_update(c, blockIdx.x, grid_blocks);
+    return;
+  }
+  if (c.ctrl->sort_active == 0 || (c.ctrl->status & 0x8u)) return;  // nothing to sort, or a bounded wait gave up
+  for (long long b = blockIdx.x - grid_blocks; b * 256 < c.n; b += gridDim.x - grid_blocks) sort_scatter(c, b);
 }
 
 // Grid heat conduction (explicit, between face-neighbour nodes that both hold mass this substep):
@@ -2228,8 +2395,10 @@ void launch_grid_clear(const Ctx& c, cudaStream_t st, int grid_blocks) {
   k_grid_clear<<<grid_blocks, 256, 0, st>>>(c);
 }
 
-void launch_grid_update(const Ctx& c, cudaStream_t st, int grid_blocks) {
-  k_grid_update<<<grid_blocks, 256, 0, st>>>(c);
+void launch_grid_sort(const Ctx& c, cudaStream_t st, int grid_blocks, int sort_blocks) {
+  const long long most = (c.n + 255) / 256;
+  const long long blocks = grid_blocks + (sort_blocks < most ? sort_blocks : most);
+  if (blocks > 0) k_grid_sort<<<static_cast<unsigned>(blocks), 256, 0, st>>>(c, static_cast<unsigned>(grid_blocks));
 }
 
 
@@ -2500,6 +2669,7 @@ void launch_upload_convert(const Ctx& c, cudaStream_t st, long long n, int dtype
 // so each tile's particles are contiguous in every array.
 __global__ void k_permute(Ctx c, Particles d) {
   const Particles& s = c.p;
+  if (blockIdx.x == 0 && threadIdx.x == 0) c.ctrl->in_place = 1u;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < c.n; i += (long long)gridDim.x * blockDim.x) {
     const unsigned h = s.perm[i];
     d.qx[i] = s.qx[h]; d.qy[i] = s.qy[h]; d.qz[i] = s.qz[h];
@@ -2526,7 +2696,7 @@ __global__ void __launch_bounds__(256) k_cell_order(Ctx c) {
   __shared__ unsigned ids[kCellSortMax];
   __shared__ unsigned char cell[kCellSortMax];
   __shared__ int cursor[64];
-  const unsigned list = c.ctrl->step_index & 1u;
+  const unsigned list = c.ctrl->sort_list;
   const unsigned nwork = min(c.ctrl->work_count[list], static_cast<unsigned>(c.total_tiles));
   for (unsigned w = blockIdx.x; w < nwork; w += gridDim.x) {
     const uint4 it = c.s.work[list][w];  // (tile, start, count, scene)
