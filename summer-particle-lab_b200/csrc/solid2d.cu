@@ -42,6 +42,11 @@ struct Ctrl2 {
   unsigned wave_bits, grad_bits;  // stableStep maxima (non-negative floats compare as uints)
   // stats reduction
   unsigned count, minj_key, maxj_key, strain_bits;
+  // k2_frame: arrivals at the grid barrier, a barrier wait that gave up, and by substep parity the
+  // stableStep maxima and the active-node count
+  unsigned barrier, timeout;
+  unsigned wave2[2], grad2[2];
+  int active2[2];
 };
 
 struct Params2 {
@@ -170,6 +175,80 @@ __global__ void __launch_bounds__(kThreads) k2_stable(Dev2 d, Params2 p) {
   if (threadIdx.x == 0) finish_stable(d.ctrl, false);
 }
 
+// The P2G scatter of one particle (src/solid-mpm.js:50-64).
+__device__ __forceinline__ void scatter2(const Dev2& d, const St2& s, const Params2& p, float h, float4 F, float4 C,
+                                         float m, float V0, float vx, float vy, bool pin) {
+  const float rho = m / V0, E = rho * 16000.f * p.stiffness;
+  float tau[4];
+  solid_stress(F.x, F.y, F.z, F.w, .4f * E, .4f * E, tau);
+  const float factor = -h * V0 * 4.f / (kDX * kDX);
+  const float a00 = m * C.x + factor * tau[0], a01 = m * C.y + factor * tau[1];
+  const float a10 = m * C.z + factor * tau[2], a11 = m * C.w + factor * tau[3];
+  const float pm = pin ? m : 0.f;
+#pragma unroll
+  for (int j = 0; j < 3; ++j)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const float w = s.wx[k] * s.wy[j], dx = ((float)k - s.fx) * kDX, dy = ((float)j - s.fy) * kDX;
+      const int n = (s.by + j) * kN + s.bx + k;
+      atomicAdd(&d.grid[n], make_float4(w * m, w * (m * vx + a00 * dx + a01 * dy), w * (m * vy + a10 * dx + a11 * dy),
+                                        w * pm));
+    }
+}
+
+// Grid update of one node (src/solid-mpm.js:65-76); clears its accumulator for the next P2G. Returns 1
+// for a node with mass.
+__device__ __forceinline__ int update_node2(const Dev2& d, const Params2& p, int n) {
+  const float4 a = __ldcg(&d.grid[n]);
+  d.grid[n] = make_float4(0.f, 0.f, 0.f, 0.f);
+  float ux = a.y, uy = a.z;  // a node at or below the mass threshold keeps its raw sums
+  int active = 0;
+  if (a.x > 1e-12f) {
+    active = 1;
+    ux /= a.x;
+    uy /= a.x;
+    if (a.w > 1e-9f) {
+      ux = uy = 0.f;
+    } else if (p.walls) {
+      const float x = kOrigin + (float)(n % kN) * kDX, y = kOrigin + (float)(n / kN) * kDX;
+      if ((x < -p.bound + kDX && ux < 0.f) || (x > p.bound - kDX && ux > 0.f)) ux = 0.f;
+      if ((y < p.floor_ + kDX && uy < 0.f) || (y > p.top - kDX && uy > 0.f)) uy = 0.f;
+    }
+  }
+  d.vel[n] = make_float2(ux, uy);
+  return active;
+}
+
+// G2P of one moving particle with the C and F update and the wall clamp (src/solid-mpm.js:77-90).
+__device__ __forceinline__ void gather2(const Dev2& d, const St2& s, const Params2& p, float h, float& x, float& y,
+                                        float& vx, float& vy, float4& F, float4& C) {
+  float gvx = 0.f, gvy = 0.f, a = 0.f, b = 0.f, c = 0.f, e = 0.f;
+#pragma unroll
+  for (int j = 0; j < 3; ++j)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const float2 u = __ldcg(&d.vel[(s.by + j) * kN + s.bx + k]);
+      const float w = s.wx[k] * s.wy[j], dx = ((float)k - s.fx) * (4.f / kDX), dy = ((float)j - s.fy) * (4.f / kDX);
+      gvx += w * u.x;
+      gvy += w * u.y;
+      a += w * u.x * dx;
+      b += w * u.x * dy;
+      c += w * u.y * dx;
+      e += w * u.y * dy;
+    }
+  C = make_float4(a, b, c, e);
+  F = make_float4((1.f + h * a) * F.x + h * b * F.z, (1.f + h * a) * F.y + h * b * F.w,
+                  h * c * F.x + (1.f + h * e) * F.z, h * c * F.y + (1.f + h * e) * F.w);
+  vx = gvx;
+  vy = gvy;
+  x += h * vx;
+  y += h * vy;
+  if (p.walls) {
+    x = fminf(fmaxf(x, -p.bound + .1f), p.bound - .1f);
+    y = fminf(fmaxf(y, p.floor_ + .1f), p.top - .1f);
+  }
+}
+
 // Body force of Simulation.substep for MPM solids (src/simulation.js:270-288, force != 0 only
 // in frame mode) and the P2G scatter of src/solid-mpm.js:50-64.
 __global__ void __launch_bounds__(kThreads) k2_p2g(Dev2 d, Params2 p, int frame) {
@@ -201,48 +280,15 @@ __global__ void __launch_bounds__(kThreads) k2_p2g(Dev2 d, Params2 p, int frame)
     }
     St2 s;
     stencil2(x, y, s);
-    const float m = d.mass[i], V0 = kArea * d.volume[i], rho = m / V0, E = rho * 16000.f * p.stiffness;
-    const float4 F = d.F[i], C = d.C[i];
-    float tau[4];
-    solid_stress(F.x, F.y, F.z, F.w, .4f * E, .4f * E, tau);
-    const float factor = -h * V0 * 4.f / (kDX * kDX);
-    const float a00 = m * C.x + factor * tau[0], a01 = m * C.y + factor * tau[1];
-    const float a10 = m * C.z + factor * tau[2], a11 = m * C.w + factor * tau[3];
-    const float pm = pin ? m : 0.f;
-#pragma unroll
-    for (int j = 0; j < 3; ++j)
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const float w = s.wx[k] * s.wy[j], dx = ((float)k - s.fx) * kDX, dy = ((float)j - s.fy) * kDX;
-        const int n = (s.by + j) * kN + s.bx + k;
-        atomicAdd(&d.grid[n], make_float4(w * m, w * (m * vx + a00 * dx + a01 * dy), w * (m * vy + a10 * dx + a11 * dy),
-                                          w * pm));
-      }
+    scatter2(d, s, p, h, d.F[i], d.C[i], d.mass[i], kArea * d.volume[i], vx, vy, pin);
   }
 }
 
-// Grid update of src/solid-mpm.js:65-76; clears the accumulator for the next P2G.
+// Grid update of every node.
 __global__ void __launch_bounds__(kThreads) k2_grid(Dev2 d, Params2 p) {
   if (d.ctrl->done) return;
   int active = 0;
-  for (int n = blockIdx.x * kThreads + threadIdx.x; n < kNodes; n += gridDim.x * kThreads) {
-    const float4 a = d.grid[n];
-    d.grid[n] = make_float4(0.f, 0.f, 0.f, 0.f);
-    float ux = a.y, uy = a.z;  // a node at or below the mass threshold keeps its raw sums
-    if (a.x > 1e-12f) {
-      ++active;
-      ux /= a.x;
-      uy /= a.x;
-      if (a.w > 1e-9f) {
-        ux = uy = 0.f;
-      } else if (p.walls) {
-        const float x = kOrigin + (float)(n % kN) * kDX, y = kOrigin + (float)(n / kN) * kDX;
-        if ((x < -p.bound + kDX && ux < 0.f) || (x > p.bound - kDX && ux > 0.f)) ux = 0.f;
-        if ((y < p.floor_ + kDX && uy < 0.f) || (y > p.top - kDX && uy > 0.f)) uy = 0.f;
-      }
-    }
-    d.vel[n] = make_float2(ux, uy);
-  }
+  for (int n = blockIdx.x * kThreads + threadIdx.x; n < kNodes; n += gridDim.x * kThreads) active += update_node2(d, p, n);
   for (int o = 16; o; o >>= 1) active += __shfl_xor_sync(0xffffffffu, active, o);
   if ((threadIdx.x & 31) == 0 && active) atomicAdd(&d.ctrl->active_nodes, active);
 }
@@ -260,31 +306,7 @@ __global__ void __launch_bounds__(kThreads) k2_g2p(Dev2 d, Params2 p, int frame)
       float x = d.x[i], y = d.y[i];
       St2 s;
       stencil2(x, y, s);
-      float gvx = 0.f, gvy = 0.f, a = 0.f, b = 0.f, c = 0.f, e = 0.f;
-#pragma unroll
-      for (int j = 0; j < 3; ++j)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          const float2 u = d.vel[(s.by + j) * kN + s.bx + k];
-          const float w = s.wx[k] * s.wy[j], dx = ((float)k - s.fx) * (4.f / kDX), dy = ((float)j - s.fy) * (4.f / kDX);
-          gvx += w * u.x;
-          gvy += w * u.y;
-          a += w * u.x * dx;
-          b += w * u.x * dy;
-          c += w * u.y * dx;
-          e += w * u.y * dy;
-        }
-      C = make_float4(a, b, c, e);
-      F = make_float4((1.f + h * a) * F.x + h * b * F.z, (1.f + h * a) * F.y + h * b * F.w,
-                      h * c * F.x + (1.f + h * e) * F.z, h * c * F.y + (1.f + h * e) * F.w);
-      vx = gvx;
-      vy = gvy;
-      x += h * vx;
-      y += h * vy;
-      if (p.walls) {
-        x = fminf(fmaxf(x, -p.bound + .1f), p.bound - .1f);
-        y = fminf(fmaxf(y, p.floor_ + .1f), p.top - .1f);
-      }
+      gather2(d, s, p, h, x, y, vx, vy, F, C);
       d.F[i] = F;
       d.C[i] = C;
       d.vx[i] = vx;
@@ -297,6 +319,114 @@ __global__ void __launch_bounds__(kThreads) k2_g2p(Dev2 d, Params2 p, int frame)
   if (frame) {
     block_max2(wave, grad, &d.ctrl->wave_bits, &d.ctrl->grad_bits);
     if (threadIdx.x == 0) finish_stable(d.ctrl, true);
+  }
+}
+
+// Grid barrier of a cooperative launch: round counts the barriers passed. Bounded: after about a second
+// of polling it reports false, and the kernel leaves.
+__device__ bool grid_barrier(Ctrl2* c, unsigned& round) {
+  __shared__ int ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(&c->barrier, 1u);
+    const unsigned target = ++round * gridDim.x;
+    ok = 0;
+    for (int i = 0; i < (1 << 21); ++i)
+      if (*(volatile unsigned*)&c->barrier >= target) {
+        ok = 1;
+        break;
+      }
+    if (!ok) atomicOr(&c->timeout, 1u);
+    __threadfence();
+  }
+  __syncthreads();
+  return ok != 0;
+}
+
+// A whole frame in one cooperative launch, one particle per thread, its state in registers: the same
+// substeps as k2_stable and the k2_p2g, k2_grid, k2_g2p sequence, separated by grid barriers. The reference's
+// 16,000 particles are bound by launches and host checks: four substeps took 47 us in 13 kernels with their gaps,
+// and each frame copied its control block back at least once more. Node sums and velocities are read from L2.
+__global__ void __launch_bounds__(kThreads) k2_frame(Dev2 d, Params2 p) {
+  Ctrl2* ct = d.ctrl;
+  const int i = blockIdx.x * kThreads + threadIdx.x;
+  const bool live = i < p.count && solid(p, d.material[i]);
+  const bool pin = live && d.pinned[i] != 0;
+  float x = 0.f, y = 0.f, vx = 0.f, vy = 0.f, m = 0.f, V0 = 1.f;
+  float4 F = make_float4(1.f, 0.f, 0.f, 1.f), C = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (live) {
+    x = d.x[i]; y = d.y[i]; vx = d.vx[i]; vy = d.vy[i];
+    m = d.mass[i];
+    V0 = kArea * d.volume[i];
+    F = d.F[i];
+    C = d.C[i];
+  }
+  unsigned wave = 0, grad = 0, round = 0;
+  if (live) stable_terms(p, F, C, vx, vy, wave, grad);
+  block_max2(wave, grad, &ct->wave2[0], &ct->grad2[0]);
+  double remaining = ct->remaining, h_last = 0.0;
+  int steps = 0;
+  if (!grid_barrier(ct, round)) return;
+  while (true) {
+    const int par = steps & 1;
+    // src/solid-mpm.js:45, src/simulation.js:250-253
+    const float wmax = fmaxf(1.f, __uint_as_float(__ldcg(&ct->wave2[par])));
+    const float gmax = __uint_as_float(__ldcg(&ct->grad2[par]));
+    const double stable = fmin(fmin(1.0 / 240, (double)(.18f * kDX / wmax)), (double)(.1f / fmaxf(1.f, gmax)));
+    const double hd = fmin(remaining, stable);
+    h_last = hd;
+    if (!(remaining > 1e-9 && steps < kMaxSubsteps)) break;
+    const float h = (float)hd;
+    if (i == 0) {  // the next substep's slots: last read two barriers ago, next written two barriers from here
+      ct->wave2[par ^ 1] = 0u;
+      ct->grad2[par ^ 1] = 0u;
+      ct->active2[par] = 0;
+    }
+    St2 s;
+    if (live) {
+      if (pin) {
+        vx = vy = 0.f;
+      } else {
+        float gx = 0.f, gy = 0.f;
+        if (p.gravity == SMPM_GRAVITY_CENTER) {
+          const float r = sqrtf(x * x + y * y + 400.f);
+          gx = -x / r;
+          gy = -y / r;
+        } else if (p.gravity == SMPM_GRAVITY_UNIFORM) {
+          gy = -1.f;
+        }
+        vx = fminf(fmaxf(vx + gx * p.force * h, -180.f), 180.f);
+        vy = fminf(fmaxf(vy + gy * p.force * h, -180.f), 180.f);
+      }
+      stencil2(x, y, s);
+      scatter2(d, s, p, h, F, C, m, V0, vx, vy, pin);
+    }
+    if (!grid_barrier(ct, round)) return;
+    int active = 0;
+    for (int n = i; n < kNodes; n += gridDim.x * kThreads) active += update_node2(d, p, n);
+    for (int o = 16; o; o >>= 1) active += __shfl_xor_sync(0xffffffffu, active, o);
+    if ((threadIdx.x & 31) == 0 && active) atomicAdd(&ct->active2[par], active);
+    if (!grid_barrier(ct, round)) return;
+    if (live && !pin) gather2(d, s, p, h, x, y, vx, vy, F, C);
+    wave = grad = 0;
+    if (live) stable_terms(p, F, C, vx, vy, wave, grad);
+    block_max2(wave, grad, &ct->wave2[par ^ 1], &ct->grad2[par ^ 1]);
+    remaining -= hd;
+    ++steps;
+    if (!grid_barrier(ct, round)) return;
+  }
+  if (live) {
+    d.x[i] = x; d.y[i] = y; d.vx[i] = vx; d.vy[i] = vy;
+    d.F[i] = F;
+    d.C[i] = C;
+  }
+  if (i == 0) {
+    ct->remaining = remaining;
+    ct->h = h_last;
+    ct->steps = steps;
+    ct->done = 1;
+    if (steps > 0) ct->active_nodes = __ldcg(&ct->active2[(steps - 1) & 1]);
   }
 }
 
@@ -343,6 +473,7 @@ struct smpm_handle {
   Dev2 d{};
   Ctrl2* host_ctrl = nullptr;  // pinned
   unsigned mask[8] = {};
+  int frame_blocks = 0;  // CTAs of k2_frame that are resident at once (0: no cooperative launch)
   int substeps = 0;  // SolidMPM.substeps: set by a frame
   int nodes = 0;     // SolidMPM.activeNodes: set by every grid pass
   std::string err;
@@ -461,6 +592,12 @@ int smpm_create(int64_t capacity, smpm_handle** out) {
     e = cudaGetLastError();
   }
   e = e ? e : cudaStreamSynchronize(h->stream);
+  int dev = 0, coop = 0, sms = 0, per_sm = 0;
+  if (e == cudaSuccess && cudaGetDevice(&dev) == cudaSuccess &&
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && coop &&
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k2_frame, kThreads, 0) == cudaSuccess)
+    h->frame_blocks = std::min(per_sm, 2) * sms;
   if (e != cudaSuccess) {
     smpm_destroy(h);
     return e == cudaErrorMemoryAllocation ? MPM_ERR_OUT_OF_MEMORY : MPM_ERR_CUDA;
@@ -571,6 +708,23 @@ int smpm_frame(smpm_handle* h, const smpm_sim* s, double dt, int32_t* substeps, 
   if (rc || (rc = upload_sim(h, s)) || (rc = set_ctrl(h, dt, 0.0))) return rc;
   const Params2 p = params_of(h, s);
   const int pb = blocks_for(s->count), gb = blocks_for(kNodes);
+  if (pb * static_cast<long long>(kThreads) >= s->count && pb <= h->frame_blocks) {
+    // one particle per thread, every CTA resident: the whole frame in one launch
+    Dev2 d = h->d;
+    Params2 q = p;
+    void* args[] = {&d, &q};
+    cudaError_t e = cudaLaunchCooperativeKernel((const void*)k2_frame, dim3(pb), dim3(kThreads), args, 0, h->stream);
+    if ((rc = h->cuda(e, "frame launch"))) return rc;
+    if ((rc = download_sim(h, s))) return rc;
+    if (h->host_ctrl->timeout) {
+      cudaMemsetAsync(h->d.grid, 0, kNodes * sizeof(float4), h->stream);
+      return h->fail(MPM_ERR_TIMEOUT, "a bounded device wait gave up (grid barrier)");
+    }
+    h->substeps = h->host_ctrl->steps;
+    if (substeps) *substeps = h->host_ctrl->steps;
+    if (advanced) *advanced = dt - h->host_ctrl->remaining;
+    return MPM_OK;
+  }
   k2_stable<<<pb, kThreads, 0, h->stream>>>(h->d, p);
   for (int launched = 0; launched < kMaxSubsteps;) {
     for (int k = 0; k < kBatch && launched < kMaxSubsteps; ++k, ++launched) {
