@@ -94,7 +94,6 @@ struct mpm_handle {
   void* gblock = nullptr;  size_t gblock_bytes = 0;   // grid + sort + control
   void* snap = nullptr;    bool snap_valid = false;  int64_t snap_n = 0;
   void* staging = nullptr; size_t staging_bytes = 0;
-  void** dptr_table = nullptr;                          // 12 device pointers for conversion
   double* ledger_partials = nullptr;
   double* ledger_out = nullptr;
   mpm::Ctrl* host_ctrl = nullptr;                        // pinned readback
@@ -237,7 +236,6 @@ static int free_device(mpm_handle* h) {
   if (h->gblock) cudaFree(h->gblock);
   if (h->snap) cudaFree(h->snap);
   if (h->staging) cudaFree(h->staging);
-  if (h->dptr_table) cudaFree(h->dptr_table);
   if (h->ledger_partials) cudaFree(h->ledger_partials);
   if (h->rblock) cudaFree(h->rblock);
   h->rblock = nullptr;
@@ -256,7 +254,6 @@ static int free_device(mpm_handle* h) {
   h->return_mode = MPM_RETURN_EXACT;
   h->ctx.learned = 0;
   h->pblock = h->gblock = h->snap = h->staging = nullptr;
-  h->dptr_table = nullptr;
   h->ledger_partials = nullptr;
   h->host_ctrl = nullptr;
   h->host_ledger = nullptr;
@@ -706,7 +703,6 @@ int mpm_create(const mpm_domain* domain, int64_t capacity, mpm_handle** out) {
   h->ctx.p.perm = h->palt.perm = static_cast<unsigned*>(h->sblock) + align_up(capacity, 64);
   if (cudaMemsetAsync(h->pblock, 0, pbytes, h->stream) != cudaSuccess) return bail(MPM_ERR_CUDA);
   if (cudaMemsetAsync(h->pblock_alt, 0, pbytes, h->stream) != cudaSuccess) return bail(MPM_ERR_CUDA);
-  if (cudaMalloc(reinterpret_cast<void**>(&h->dptr_table), 16 * sizeof(void*)) != cudaSuccess) return bail(MPM_ERR_OUT_OF_MEMORY);
   if (cudaMallocHost(reinterpret_cast<void**>(&h->host_ctrl), sizeof(mpm::Ctrl)) != cudaSuccess) return bail(MPM_ERR_OUT_OF_MEMORY);
   if (cudaMallocHost(reinterpret_cast<void**>(&h->host_ledger), 32 * sizeof(double)) != cudaSuccess) return bail(MPM_ERR_OUT_OF_MEMORY);
   const int ledger_blocks = h->num_sms * 4;
@@ -817,10 +813,10 @@ static int ensure_staging(mpm_handle* h, size_t bytes) {
 // Copies the caller's host arrays into device staging; fills ptrs with device addresses (or null).
 // Staged arrays: 0-2 x, y, z; 3-5 v; 6 mass; 7 volume; 8 T; 9 plastic; 10 F; 11 C; 12 Jp; 13 dilation;
 // 14 enthalpy.
-constexpr int kStaged = 15;
+constexpr int kStaged = mpm::kStagedArrays;
 static inline int staged_comps(int k) { return k == 10 || k == 11 ? 9 : 1; }
 
-static int stage_in(mpm_handle* h, int64_t n, const mpm_particles* p, void* ptrs[kStaged], const int** mat_dev,
+static int stage_in(mpm_handle* h, int64_t n, const mpm_particles* p, mpm::StagedPtrs& staged, const int** mat_dev,
                     const unsigned char** pin_dev, unsigned fields, const unsigned char** melt_dev = nullptr) {
   const size_t es = p->dtype == MPM_F32 ? 4 : 8;
   const void* src[kStaged] = {p->x, p->y, p->z, p->vx, p->vy, p->vz, p->mass, p->volume, p->temperature, p->plastic,
@@ -839,6 +835,7 @@ static int stage_in(mpm_handle* h, int64_t n, const mpm_particles* p, void* ptrs
   if (rc != MPM_OK) return rc;
   char* base = static_cast<char*>(h->staging);
   size_t off = 0;
+  void** ptrs = staged.p;
   for (int k = 0; k < kStaged; ++k) {
     ptrs[k] = nullptr;
     if (!src[k] || !(fields & need[k])) continue;
@@ -865,7 +862,6 @@ static int stage_in(mpm_handle* h, int64_t n, const mpm_particles* p, void* ptrs
     MPM_CUDA(h, cudaMemcpyAsync(base + off, p->melted, n, cudaMemcpyHostToDevice, h->stream));
     off += align_up(n, 256);
   }
-  MPM_CUDA(h, cudaMemcpyAsync(h->dptr_table, ptrs, kStaged * sizeof(void*), cudaMemcpyHostToDevice, h->stream));
   return MPM_OK;
 }
 
@@ -910,7 +906,7 @@ int mpm_upload_particles(mpm_handle* h, int64_t n, const mpm_particles* p) {
   (void)es;
   MPM_CUDA(h, cudaStreamSynchronize(h->stream));
   drop_graph(h);  // a captured graph holds the old particle count
-  void* ptrs[kStaged];
+  mpm::StagedPtrs ptrs{};
   const int* mat_dev;
   const unsigned char* pin_dev;
   const unsigned char* melt_dev;
@@ -926,7 +922,7 @@ int mpm_upload_particles(mpm_handle* h, int64_t n, const mpm_particles* p) {
   if (h->batch) {
     // scene table already on the device (alloc_grid); each particle takes its scene's material
     { ProfScope ps(h, -1);
-      mpm::launch_upload_convert(h->ctx, h->stream, n, p->dtype, reinterpret_cast<const void* const*>(h->dptr_table),
+      mpm::launch_upload_convert(h->ctx, h->stream, n, p->dtype, ptrs,
                                  nullptr, pin_dev, all, false, melt_dev); }
     MPM_CUDA(h, cudaGetLastError());
     h->n = n;
@@ -948,7 +944,7 @@ int mpm_upload_particles(mpm_handle* h, int64_t n, const mpm_particles* p) {
   tmp.mat_base = 0;
   MPM_CUDA(h, cudaMemcpyAsync(const_cast<SceneDev*>(h->ctx.scenes), &tmp, sizeof(SceneDev), cudaMemcpyHostToDevice, h->stream));
   { ProfScope ps(h, -1);
-    mpm::launch_upload_convert(h->ctx, h->stream, n, p->dtype, reinterpret_cast<const void* const*>(h->dptr_table), mat_dev,
+    mpm::launch_upload_convert(h->ctx, h->stream, n, p->dtype, ptrs, mat_dev,
                                pin_dev, all, false, melt_dev); }
   MPM_CUDA(h, cudaGetLastError());
   MPM_CUDA(h, cudaMemcpyAsync(const_cast<SceneDev*>(h->ctx.scenes), &h->scene, sizeof(SceneDev), cudaMemcpyHostToDevice,
@@ -992,7 +988,8 @@ int mpm_download_particles(mpm_handle* h, const mpm_particles* p) {
   if (p->melted) total += align_up(n, 256);
   int rc = ensure_staging(h, std::max<size_t>(total, 256));
   if (rc != MPM_OK) return rc;
-  void* dev[kStaged];
+  mpm::StagedPtrs staged{};
+  void** dev = staged.p;
   char* base = static_cast<char*>(h->staging);
   size_t off = 0;
   for (int k = 0; k < kStaged; ++k) {
@@ -1001,8 +998,7 @@ int mpm_download_particles(mpm_handle* h, const mpm_particles* p) {
     dev[k] = base + off;
     off += align_up(staged_comps(k) * n * es, 256);
   }
-  MPM_CUDA(h, cudaMemcpyAsync(h->dptr_table, dev, kStaged * sizeof(void*), cudaMemcpyHostToDevice, h->stream));
-  { ProfScope ps(h, -1); mpm::launch_download_convert(h->ctx, h->stream, n, p->dtype, reinterpret_cast<void* const*>(h->dptr_table), fields); }
+  { ProfScope ps(h, -1); mpm::launch_download_convert(h->ctx, h->stream, n, p->dtype, staged, fields); }
   MPM_CUDA(h, cudaGetLastError());
   for (int k = 0; k < kStaged; ++k)
     if (dst[k]) MPM_CUDA(h, cudaMemcpyAsync(dst[k], dev[k], staged_comps(k) * n * es, cudaMemcpyDeviceToHost, h->stream));
@@ -1350,14 +1346,14 @@ int mpm_step_host(mpm_handle* h, const mpm_particles* io, double dt) {
     return fail(h, MPM_ERR_INVALID_ARG, "positions and velocities are required");
   const int64_t n = h->n;
   if (n == 0) return MPM_OK;
-  void* ptrs[kStaged];
+  mpm::StagedPtrs ptrs{};
   const int* mat_dev;
   const unsigned char* pin_dev;
   const unsigned fields = mpm::kFieldPos | mpm::kFieldVel;
   int rc = stage_in(h, n, io, ptrs, &mat_dev, &pin_dev, fields);
   if (rc != MPM_OK) return rc;
   { ProfScope ps(h, -1);
-    mpm::launch_upload_convert(h->ctx, h->stream, n, io->dtype, reinterpret_cast<const void* const*>(h->dptr_table), nullptr,
+    mpm::launch_upload_convert(h->ctx, h->stream, n, io->dtype, ptrs, nullptr,
                                nullptr, fields, true); }
   MPM_CUDA(h, cudaGetLastError());
   rc = prepare_grid(h);
@@ -1385,14 +1381,14 @@ int mpm_frame_host(mpm_handle* h, const mpm_particles* io, double dt_requested, 
     return fail(h, MPM_ERR_INVALID_ARG, "positions and velocities are required");
   const int64_t n = h->n;
   if (n == 0) return MPM_OK;
-  void* ptrs[kStaged];
+  mpm::StagedPtrs ptrs{};
   const int* mat_dev;
   const unsigned char* pin_dev;
   const unsigned fields = mpm::kFieldPos | mpm::kFieldVel;
   int rc = stage_in(h, n, io, ptrs, &mat_dev, &pin_dev, fields);
   if (rc != MPM_OK) return rc;
   { ProfScope ps(h, -1);
-    mpm::launch_upload_convert(h->ctx, h->stream, n, io->dtype, reinterpret_cast<const void* const*>(h->dptr_table), nullptr,
+    mpm::launch_upload_convert(h->ctx, h->stream, n, io->dtype, ptrs, nullptr,
                                nullptr, fields, true); }
   MPM_CUDA(h, cudaGetLastError());
   h->grid_valid = false;
@@ -1517,13 +1513,13 @@ int mpm_regularize_host(mpm_handle* h, const mpm_particles* io, double dt) {
   if (!io->x || !io->y || !io->z) return fail(h, MPM_ERR_INVALID_ARG, "positions are required");
   if (!(dt > 0) || !std::isfinite(dt)) return fail(h, MPM_ERR_INVALID_ARG, "dt must be positive");
   if (!h->reg.enabled || h->n == 0) return MPM_OK;
-  void* ptrs[kStaged];
+  mpm::StagedPtrs ptrs{};
   const int* mat_dev;
   const unsigned char* pin_dev;
   int rc = stage_in(h, h->n, io, ptrs, &mat_dev, &pin_dev, mpm::kFieldPos);
   if (rc != MPM_OK) return rc;
   { ProfScope ps(h, -1);
-    mpm::launch_upload_convert(h->ctx, h->stream, h->n, io->dtype, reinterpret_cast<const void* const*>(h->dptr_table),
+    mpm::launch_upload_convert(h->ctx, h->stream, h->n, io->dtype, ptrs,
                                nullptr, nullptr, mpm::kFieldPos, true); }
   MPM_CUDA(h, cudaGetLastError());
   rc = regularize_now(h, nullptr, dt);

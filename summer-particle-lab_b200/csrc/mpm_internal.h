@@ -224,11 +224,16 @@ void launch_halo_add(const Ctx& c, cudaStream_t st, int side, int planes, const 
 void launch_g2p2g(const Ctx& c, cudaStream_t st, int grid_blocks, bool scatter);
 void launch_ledger(const Ctx& c, cudaStream_t st, double* partials, int blocks, double* out);
 void launch_grid_debug(const Ctx& c, cudaStream_t st, int scene, float dt, double* mass, double* mom);
-void launch_upload_convert(const Ctx& c, cudaStream_t st, long long n, int dtype, const void* const* src,
+// Device addresses of the staged arrays of an upload or download (order in mpm_api.cu), by value.
+constexpr int kStagedArrays = 15;
+struct StagedPtrs {
+  void* p[kStagedArrays];
+};
+void launch_upload_convert(const Ctx& c, cudaStream_t st, long long n, int dtype, const StagedPtrs& src,
                            const int* material, const unsigned char* pinned, unsigned fields, bool by_id,
                            const unsigned char* melted = nullptr);
 void launch_download_melted(const Ctx& c, cudaStream_t st, long long n, unsigned char* out);
-void launch_download_convert(const Ctx& c, cudaStream_t st, long long n, int dtype, void* const* dst,
+void launch_download_convert(const Ctx& c, cudaStream_t st, long long n, int dtype, const StagedPtrs& dst,
                              unsigned fields);
 void launch_permute(const Ctx& c, const Particles& dst, cudaStream_t st);
 // viewer frame: sampled rows (8 floats) and energy / temperature-range / per-material reductions

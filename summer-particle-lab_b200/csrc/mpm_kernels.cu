@@ -2580,9 +2580,12 @@ void launch_grid_debug(const Ctx& c, cudaStream_t st, int scene, float dt, doubl
 // Host arrays (staged on the device) into the SoA state. A full upload sets the home order to the
 // caller's order (id = i); with by_id the caller's particle id[i] is read into home slot i.
 template <typename Tsrc>
-__global__ void k_upload(Ctx c, long long n, const Tsrc* const* src, const int* material,
+__global__ void k_upload(Ctx c, long long n, const __grid_constant__ StagedPtrs arrays, const int* material,
                          const unsigned char* pinned, unsigned fields, int by_id, const unsigned char* melted) {
   const long long cap = c.p.cap;
+  const Tsrc* src[kStagedArrays];
+#pragma unroll
+  for (int k = 0; k < kStagedArrays; ++k) src[k] = static_cast<const Tsrc*>(arrays.p[k]);
   for (long long h = blockIdx.x * (long long)blockDim.x + threadIdx.x; h < n; h += (long long)gridDim.x * blockDim.x) {
     const long long i = by_id ? (long long)c.p.id[h] : h;
     if (!by_id) c.p.id[h] = static_cast<unsigned>(h);
@@ -2590,6 +2593,7 @@ __global__ void k_upload(Ctx c, long long n, const Tsrc* const* src, const int* 
     const SceneDev& sc = c.scenes[s];
     if (fields & kFieldPos) {
       unsigned* qs[3] = {c.p.qx, c.p.qy, c.p.qz};
+#pragma unroll
       for (int a = 0; a < 3; ++a) {
         const double q = rint(((double)src[a][i] - sc.origin[a]) / (double)sc.H * 4194304.0);
         const double hi = (double)(((long long)sc.dims[a] - 1) << kFracBits);
@@ -2652,16 +2656,16 @@ __global__ void k_upload(Ctx c, long long n, const Tsrc* const* src, const int* 
   }
 }
 
-void launch_upload_convert(const Ctx& c, cudaStream_t st, long long n, int dtype, const void* const* src,
+void launch_upload_convert(const Ctx& c, cudaStream_t st, long long n, int dtype, const StagedPtrs& src,
                            const int* material, const unsigned char* pinned, unsigned fields, bool by_id,
                            const unsigned char* melted) {
   if (n <= 0) return;
   const int blocks = static_cast<int>((n + 255) / 256 < 65536 ? (n + 255) / 256 : 65536);
   if (dtype == 0)
-    k_upload<double><<<blocks, 256, 0, st>>>(c, n, reinterpret_cast<const double* const*>(src), material, pinned, fields,
+    k_upload<double><<<blocks, 256, 0, st>>>(c, n, src, material, pinned, fields,
                                              by_id ? 1 : 0, melted);
   else
-    k_upload<float><<<blocks, 256, 0, st>>>(c, n, reinterpret_cast<const float* const*>(src), material, pinned, fields,
+    k_upload<float><<<blocks, 256, 0, st>>>(c, n, src, material, pinned, fields,
                                             by_id ? 1 : 0, melted);
 }
 
@@ -2800,14 +2804,18 @@ void launch_edit_particle(const Ctx& c, cudaStream_t st, int op, unsigned a, con
 }
 
 template <typename Tdst>
-__global__ void k_download(Ctx c, long long n, Tdst* const* dst, unsigned fields) {
+__global__ void k_download(Ctx c, long long n, const __grid_constant__ StagedPtrs arrays, unsigned fields) {
   const long long cap = c.p.cap;
+  Tdst* dst[kStagedArrays];
+#pragma unroll
+  for (int k = 0; k < kStagedArrays; ++k) dst[k] = static_cast<Tdst*>(arrays.p[k]);
   for (long long h = blockIdx.x * (long long)blockDim.x + threadIdx.x; h < n; h += (long long)gridDim.x * blockDim.x) {
     const long long i = c.p.id[h];  // caller's index of home slot h
     const int s = c.nscenes == 1 ? 0 : find_scene_by_particle(c.scenes, c.nscenes, h);
     const SceneDev& sc = c.scenes[s];
     if (fields & kFieldPos) {
       const unsigned q[3] = {c.p.qx[h], c.p.qy[h], c.p.qz[h]};
+#pragma unroll
       for (int a = 0; a < 3; ++a) dst[a][i] = (Tdst)(sc.origin[a] + (double)q[a] * ((double)sc.H / 4194304.0));
     }
     if (fields & kFieldVel) {
@@ -2850,13 +2858,13 @@ void launch_download_melted(const Ctx& c, cudaStream_t st, long long n, unsigned
   k_download_melted<<<blocks, 256, 0, st>>>(c, n, out);
 }
 
-void launch_download_convert(const Ctx& c, cudaStream_t st, long long n, int dtype, void* const* dst, unsigned fields) {
+void launch_download_convert(const Ctx& c, cudaStream_t st, long long n, int dtype, const StagedPtrs& dst, unsigned fields) {
   if (n <= 0) return;
   const int blocks = static_cast<int>((n + 255) / 256 < 65536 ? (n + 255) / 256 : 65536);
   if (dtype == 0)
-    k_download<double><<<blocks, 256, 0, st>>>(c, n, reinterpret_cast<double* const*>(dst), fields);
+    k_download<double><<<blocks, 256, 0, st>>>(c, n, dst, fields);
   else
-    k_download<float><<<blocks, 256, 0, st>>>(c, n, reinterpret_cast<float* const*>(dst), fields);
+    k_download<float><<<blocks, 256, 0, st>>>(c, n, dst, fields);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -31,6 +31,8 @@ constexpr float kDX = 8.f, kOrigin = -592.f, kArea = 12.96f;
 constexpr int kThreads = 128;
 constexpr int kMaxSubsteps = 96;  // src/simulation.js:250
 constexpr int kBatch = 4;         // substeps launched per host check
+constexpr size_t kCtrlBytes = 256;       // the control block's place before the particle arrays
+constexpr long long kStageCount = 65536;  // calls of up to this many particles are staged
 
 struct Ctrl2 {
   double remaining;  // frame time still to solve
@@ -471,7 +473,8 @@ struct smpm_handle {
   long long capacity = 0;
   cudaStream_t stream = nullptr;
   Dev2 d{};
-  Ctrl2* host_ctrl = nullptr;  // pinned
+  Ctrl2* host_ctrl = nullptr;  // pinned: the control block, then room for the arrays of a staged call
+  size_t stage_bytes = 0;      // size of that block
   unsigned mask[8] = {};
   int frame_blocks = 0;  // CTAs of k2_frame that are resident at once (0: no cooperative launch)
   int substeps = 0;  // SolidMPM.substeps: set by a frame
@@ -518,45 +521,80 @@ Params2 params_of(const smpm_handle* h, const smpm_sim* s) {
   return p;
 }
 
-int upload_sim(smpm_handle* h, const smpm_sim* s) {
-  const size_t n = (size_t)s->count;
-  if (!n) return MPM_OK;
-  cudaStream_t st = h->stream;
-  const size_t f = n * sizeof(float);
+// The call's particle arrays follow the control block in one device block, packed for the count: x, y, vx
+// and vy, which come back, then mass, volume, material and pinned. Returns the bytes up to vy's end.
+size_t lay_out(smpm_handle* h, size_t n, size_t* total) {
+  char* base = reinterpret_cast<char*>(h->d.ctrl);
+  size_t off = kCtrlBytes;
+  auto take = [&](size_t bytes) {
+    char* at = base + off;
+    off += (bytes + 15) & ~size_t(15);
+    return at;
+  };
+  float** fl[6] = {&h->d.x, &h->d.y, &h->d.vx, &h->d.vy, &h->d.mass, &h->d.volume};
+  size_t back = 0;
+  for (int k = 0; k < 6; ++k) {
+    *fl[k] = reinterpret_cast<float*>(take(n * sizeof(float)));
+    if (k == 3) back = off;
+  }
+  h->d.material = reinterpret_cast<uint8_t*>(take(n));
+  h->d.pinned = reinterpret_cast<uint8_t*>(take(n));
+  *total = off;
+  return back;
+}
+
+Ctrl2 ctrl_of(double remaining, double step) {
+  Ctrl2 c{};
+  c.remaining = remaining;
+  c.h = step;
+  c.minj_key = 0xffffffffu;
+  return c;
+}
+
+// The control block and the caller's arrays to the device. Up to the pinned block's size they go through it as
+// one copy: eight copies of pageable arrays and their staging in the driver were most of a frame's host time.
+// The block is read again only after the call's last synchronisation.
+int upload_sim(smpm_handle* h, const smpm_sim* s, double remaining, double step) {
+  const size_t n = (size_t)s->count, f = n * sizeof(float);
+  size_t total = 0;
+  lay_out(h, n, &total);
+  const void* src[8] = {s->x, s->y, s->vx, s->vy, s->mass, s->volume, s->material, s->pinned};
+  void* dst[8] = {h->d.x, h->d.y, h->d.vx, h->d.vy, h->d.mass, h->d.volume, h->d.material, h->d.pinned};
+  char* dev = reinterpret_cast<char*>(h->d.ctrl);
+  *h->host_ctrl = ctrl_of(remaining, step);
   cudaError_t e = cudaSuccess;
-  e = e ? e : cudaMemcpyAsync(h->d.x, s->x, f, cudaMemcpyHostToDevice, st);
-  e = e ? e : cudaMemcpyAsync(h->d.y, s->y, f, cudaMemcpyHostToDevice, st);
-  e = e ? e : cudaMemcpyAsync(h->d.vx, s->vx, f, cudaMemcpyHostToDevice, st);
-  e = e ? e : cudaMemcpyAsync(h->d.vy, s->vy, f, cudaMemcpyHostToDevice, st);
-  e = e ? e : cudaMemcpyAsync(h->d.mass, s->mass, f, cudaMemcpyHostToDevice, st);
-  e = e ? e : cudaMemcpyAsync(h->d.volume, s->volume, f, cudaMemcpyHostToDevice, st);
-  e = e ? e : cudaMemcpyAsync(h->d.material, s->material, n, cudaMemcpyHostToDevice, st);
-  e = e ? e : cudaMemcpyAsync(h->d.pinned, s->pinned, n, cudaMemcpyHostToDevice, st);
+  if (total <= h->stage_bytes) {
+    char* host = reinterpret_cast<char*>(h->host_ctrl);
+    for (int k = 0; k < 8 && n; ++k) std::memcpy(host + (static_cast<char*>(dst[k]) - dev), src[k], k < 6 ? f : n);
+    e = cudaMemcpyAsync(dev, host, total, cudaMemcpyHostToDevice, h->stream);
+    return h->cuda(e, "copy particles in");
+  }
+  e = cudaMemcpyAsync(dev, h->host_ctrl, sizeof(Ctrl2), cudaMemcpyHostToDevice, h->stream);
+  for (int k = 0; k < 8; ++k) e = e ? e : cudaMemcpyAsync(dst[k], src[k], k < 6 ? f : n, cudaMemcpyHostToDevice, h->stream);
+  e = e ? e : cudaStreamSynchronize(h->stream);
   return h->cuda(e, "copy particles in");
 }
 
 int download_sim(smpm_handle* h, const smpm_sim* s) {
-  const size_t f = (size_t)s->count * sizeof(float);
-  cudaStream_t st = h->stream;
-  cudaError_t e = cudaSuccess;
-  if (f) {
-    e = e ? e : cudaMemcpyAsync(s->x, h->d.x, f, cudaMemcpyDeviceToHost, st);
-    e = e ? e : cudaMemcpyAsync(s->y, h->d.y, f, cudaMemcpyDeviceToHost, st);
-    e = e ? e : cudaMemcpyAsync(s->vx, h->d.vx, f, cudaMemcpyDeviceToHost, st);
-    e = e ? e : cudaMemcpyAsync(s->vy, h->d.vy, f, cudaMemcpyDeviceToHost, st);
-  }
-  e = e ? e : cudaMemcpyAsync(h->host_ctrl, h->d.ctrl, sizeof(Ctrl2), cudaMemcpyDeviceToHost, st);
-  e = e ? e : cudaStreamSynchronize(st);
+  const size_t n = (size_t)s->count, f = n * sizeof(float);
+  size_t total = 0;
+  const size_t back = lay_out(h, n, &total);
+  float* dst[4] = {s->x, s->y, s->vx, s->vy};
+  float* src[4] = {h->d.x, h->d.y, h->d.vx, h->d.vy};
+  char* dev = reinterpret_cast<char*>(h->d.ctrl);
+  char* host = reinterpret_cast<char*>(h->host_ctrl);
+  const bool staged = total <= h->stage_bytes;
+  cudaError_t e = cudaMemcpyAsync(host, dev, staged ? back : sizeof(Ctrl2), cudaMemcpyDeviceToHost, h->stream);
+  for (int k = 0; k < 4 && !staged; ++k) e = e ? e : cudaMemcpyAsync(dst[k], src[k], f, cudaMemcpyDeviceToHost, h->stream);
+  e = e ? e : cudaStreamSynchronize(h->stream);
+  if (e == cudaSuccess && staged && n)
+    for (int k = 0; k < 4; ++k) std::memcpy(dst[k], host + (reinterpret_cast<char*>(src[k]) - dev), f);
   if (e == cudaSuccess) h->nodes = h->host_ctrl->active_nodes;
   return h->cuda(e, "copy particles out");
 }
 
 int set_ctrl(smpm_handle* h, double remaining, double step) {
-  Ctrl2 c{};
-  c.remaining = remaining;
-  c.h = step;
-  c.minj_key = 0xffffffffu;
-  *h->host_ctrl = c;
+  *h->host_ctrl = ctrl_of(remaining, step);
   cudaError_t e = cudaMemcpyAsync(h->d.ctrl, h->host_ctrl, sizeof(Ctrl2), cudaMemcpyHostToDevice, h->stream);
   // the pinned block is rewritten by the next read-back only after this copy completes
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
@@ -577,14 +615,13 @@ int smpm_create(int64_t capacity, smpm_handle** out) {
   cudaError_t e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
   e = e ? e : cudaMalloc(&h->d.F, n * sizeof(float4));
   e = e ? e : cudaMalloc(&h->d.C, n * sizeof(float4));
-  float** fl[6] = {&h->d.x, &h->d.y, &h->d.vx, &h->d.vy, &h->d.mass, &h->d.volume};
-  for (float** a : fl) e = e ? e : cudaMalloc(a, n * sizeof(float));
-  e = e ? e : cudaMalloc(&h->d.material, n);
-  e = e ? e : cudaMalloc(&h->d.pinned, n);
+  static_assert(sizeof(Ctrl2) <= kCtrlBytes, "control block");
+  auto block = [](size_t count) { return kCtrlBytes + 6 * ((count * sizeof(float) + 15) & ~size_t(15)) + 2 * ((count + 15) & ~size_t(15)); };
+  h->stage_bytes = block((size_t)std::min<long long>(capacity, kStageCount));
   e = e ? e : cudaMalloc(&h->d.grid, kNodes * sizeof(float4));
   e = e ? e : cudaMalloc(&h->d.vel, kNodes * sizeof(float2));
-  e = e ? e : cudaMalloc(&h->d.ctrl, sizeof(Ctrl2));
-  e = e ? e : cudaMallocHost(&h->host_ctrl, sizeof(Ctrl2));
+  e = e ? e : cudaMalloc(&h->d.ctrl, block(n));
+  e = e ? e : cudaMallocHost(&h->host_ctrl, h->stage_bytes);
   e = e ? e : cudaMemsetAsync(h->d.grid, 0, kNodes * sizeof(float4), h->stream);
   e = e ? e : cudaMemsetAsync(h->d.ctrl, 0, sizeof(Ctrl2), h->stream);
   if (e == cudaSuccess) {
@@ -609,8 +646,7 @@ int smpm_create(int64_t capacity, smpm_handle** out) {
 int smpm_destroy(smpm_handle* h) {
   if (!h) return MPM_ERR_INVALID_ARG;
   if (h->stream) cudaStreamSynchronize(h->stream);
-  void* bufs[] = {h->d.F, h->d.C, h->d.x, h->d.y, h->d.vx, h->d.vy, h->d.mass, h->d.volume,
-                  h->d.material, h->d.pinned, h->d.grid, h->d.vel, h->d.ctrl};
+  void* bufs[] = {h->d.F, h->d.C, h->d.grid, h->d.vel, h->d.ctrl};
   for (void* b : bufs)
     if (b) cudaFree(b);
   if (h->host_ctrl) cudaFreeHost(h->host_ctrl);
@@ -674,7 +710,7 @@ int smpm_has_particles(smpm_handle* h, const smpm_sim* s, int32_t* out) {
 int smpm_stable_step(smpm_handle* h, const smpm_sim* s, double* dt) {
   if (!h || !dt) return MPM_ERR_INVALID_ARG;
   int rc = check_sim(h, s);
-  if (rc || (rc = upload_sim(h, s)) || (rc = set_ctrl(h, INFINITY, 0.0))) return rc;
+  if (rc || (rc = upload_sim(h, s, INFINITY, 0.0))) return rc;
   const Params2 p = params_of(h, s);
   k2_stable<<<blocks_for(s->count), kThreads, 0, h->stream>>>(h->d, p);
   cudaError_t e = cudaGetLastError();
@@ -689,7 +725,7 @@ int smpm_step(smpm_handle* h, const smpm_sim* s, double dt) {
   if (!h) return MPM_ERR_INVALID_ARG;
   if (!std::isfinite(dt) || dt < 0) return h->fail(MPM_ERR_INVALID_ARG, "dt must be finite and >= 0");
   int rc = check_sim(h, s);
-  if (rc || (rc = upload_sim(h, s)) || (rc = set_ctrl(h, dt, dt))) return rc;
+  if (rc || (rc = upload_sim(h, s, dt, dt))) return rc;
   const Params2 p = params_of(h, s);
   k2_p2g<<<blocks_for(s->count), kThreads, 0, h->stream>>>(h->d, p, 0);
   k2_grid<<<blocks_for(kNodes), kThreads, 0, h->stream>>>(h->d, p);
@@ -705,7 +741,7 @@ int smpm_frame(smpm_handle* h, const smpm_sim* s, double dt, int32_t* substeps, 
     return h->fail(MPM_ERR_UNSUPPORTED, "gravity mode not supported by the MPM frame");
   int rc = check_sim(h, s);
   dt = std::min(std::max(dt, 0.0), 0.05);  // src/simulation.js:241
-  if (rc || (rc = upload_sim(h, s)) || (rc = set_ctrl(h, dt, 0.0))) return rc;
+  if (rc || (rc = upload_sim(h, s, dt, 0.0))) return rc;
   const Params2 p = params_of(h, s);
   const int pb = blocks_for(s->count), gb = blocks_for(kNodes);
   if (pb * static_cast<long long>(kThreads) >= s->count && pb <= h->frame_blocks) {
@@ -749,6 +785,8 @@ int smpm_stats_get(smpm_handle* h, const smpm_sim* s, smpm_stats* out) {
   if (!h || !out) return MPM_ERR_INVALID_ARG;
   int rc = check_sim(h, s);
   if (rc) return rc;
+  size_t total = 0;
+  lay_out(h, (size_t)s->count, &total);
   if (s->count > 0) {
     cudaError_t e = cudaMemcpyAsync(h->d.material, s->material, (size_t)s->count, cudaMemcpyHostToDevice, h->stream);
     if ((rc = h->cuda(e, "stats input"))) return rc;
