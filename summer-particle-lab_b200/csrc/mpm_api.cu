@@ -25,6 +25,7 @@ namespace {
 
 constexpr int kMaxMats = 256;
 constexpr uint32_t kCheckpointMagic = 0x3242504du;  // "MPB2"
+constexpr int kMinSplitShift = 8;  // see split_shift
 constexpr uint32_t kCheckpointVersion = 3;  // 2: home-slot id array saved; 3: aux (Jp / dilation) saved
 
 size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
@@ -348,8 +349,10 @@ static int alloc_grid(mpm_handle* h) {
     c.s.block_off = cv.take<unsigned>(scan_blocks + 1);
     c.s.rank = cv.take<unsigned>(tiles + 1);
     c.s.block_rank = cv.take<unsigned>(scan_blocks + 1);
-    c.s.work[0] = cv.take<uint4>(tiles);
-    c.s.work[1] = cv.take<uint4>(tiles);
+    // every non-empty tile, and one more item for each full 2^kMinSplitShift particles
+    c.s.work_cap = static_cast<unsigned>(tiles + (h->cap >> kMinSplitShift) + 1);
+    c.s.work[0] = cv.take<uint4>(c.s.work_cap);
+    c.s.work[1] = cv.take<uint4>(c.s.work_cap);
     c.ctrl = cv.take<mpm::Ctrl>(1);
     c.dt_scene = cv.take<float>(ns);
     c.wave_max = cv.take<unsigned>(ns);
@@ -461,11 +464,22 @@ static int check_status(mpm_handle* h) {
   return status_error(h, h->host_ctrl->status);
 }
 
+// Particles per work item of the particle pass, as a power of two (31: whole tiles). A tile costs a CTA about
+// 9 us whatever it holds, so tiles are split only while the parts still find CTAs of their own: 256
+// particles (one round of phase A) up to as many as the resident CTAs hold at that size. Substep at 13,824
+// particles 33.1 -> 27.8 us, at 45,448 34.1 -> 29.9, at 131,072 47.5 -> 48.9 (so not split). The history laws' long
+// phase A moves the line: 171,360 particles of soil 81.9 -> 77.5 us.
+static int split_shift(const mpm_handle* h) {
+  const int64_t resident = static_cast<int64_t>(h->p2g_blocks) << kMinSplitShift;
+  return h->n <= resident * (h->ctx.has_aux ? 3 : 1) ? kMinSplitShift : 31;
+}
+
 // Counting sort of the current state by tile and the dt-free P2G into acc[step_index & 1].
 static int prepare_grid(mpm_handle* h) {
   h->sort_pending = false;  // everything is sorted anew (the counts are cleared below)
   Ctx& c = h->ctx;
   c.n = h->n;
+  c.split_shift = split_shift(h);
   if (h->pending_grid) {
     ProfScope ps(h, -1);
     mpm::launch_grid_clear(c, h->stream, h->grid_blocks);

@@ -39,9 +39,10 @@ constexpr int kBlock = 256;                      // threads per CTA in the parti
 constexpr int kMaxScenes = 4096;
 constexpr int kMaxMaterials = 4096;
 
-// Largest tile count whose scan k_open does by itself (3 us per 4,096 tiles, in the few substeps that sort);
-// above it k_scan is launched, about 2 us in every substep.
-constexpr int kOpenScanTiles = 16384;
+// Largest tile count whose scan k_open does by itself, in the few substeps that sort; above it k_scan is
+// launched in every substep. Substep at 110,592 particles and 32,768 tiles, k_scan against k_open: at rest 43.1 and
+// 40.3 us, at .02 cells a substep 50.4 and 50.5, at .3 cells (sorted every time) 53.5 and 57.2.
+constexpr int kOpenScanTiles = 32768;
 
 enum StepMode : int { kModeFixed = 0, kModeRequested = 1, kModeCfl = 2 };
 
@@ -137,9 +138,10 @@ struct SortBufs {
   unsigned* count;      // per particle tile, total_tiles + 1
   unsigned* start;      // block-local exclusive scan, total_tiles + 1
   unsigned* block_off;  // exclusive scan of block sums
-  unsigned* rank;       // block-local exclusive count of non-empty tiles before each tile
-  unsigned* block_rank; // exclusive scan of the blocks' non-empty tile counts
-  uint4* work[2];       // (tile, start, count, scene), non-empty tiles in tile-key order
+  unsigned* rank;       // block-local exclusive count of work items before each tile
+  unsigned* block_rank; // exclusive scan of the blocks' item counts
+  uint4* work[2];       // (tile, start, count, scene): the non-empty tiles, in parts, in tile-key order
+  unsigned work_cap;    // entries each list holds
 };
 
 struct Ctx {
@@ -165,6 +167,7 @@ struct Ctx {
   int has_thermal;      // temperature array is read and written
   int has_plastic;      // plastic strain array is read and written
   int has_aux;          // aux array is read and written (a snow, sand or pressure material is set)
+  int split_shift;      // a work item holds at most 2^split_shift particles
   int force_sort;       // this scatter pass writes keys whatever sort_want says
   int use_tma;
   int ws_blocks;        // > 0: the particle passes that scatter run warp-specialised on this many CTAs

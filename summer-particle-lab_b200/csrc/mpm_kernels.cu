@@ -368,8 +368,8 @@ constexpr int kScanPer = 4;
 constexpr int kScanChunk = kScanThreads * kScanPer;  // 4096 tiles per block
 
 // Exclusive scans of count[0..T] into start (block-local) + block_off (per 4096 tiles), and of the
-// non-empty flags into rank + block_rank (a tile's place in the work list, which so comes out in
-// tile-key order). The last block to finish scans the block sums (threadfence + ticket) and sets
+// tiles' item counts into rank + block_rank (a tile's place in the work list, which so comes out in
+// tile-key order; an empty tile has none). The last block to finish scans the block sums (threadfence + ticket) and sets
 // the work list's length.
 // The new list becomes the one that passes read. initial: a first sort; otherwise after a scatter pass,
 // if it wrote keys.
@@ -386,6 +386,9 @@ __device__ __forceinline__ uint2 warp_incl_scan2(uint2 v, int lane) {
   return v;
 }
 
+// Work items of a tile with cnt particles (0 for an empty tile).
+__device__ __forceinline__ unsigned tile_items(unsigned cnt, int shift) { return (cnt + (1u << shift) - 1u) >> shift; }
+
 __global__ void __launch_bounds__(kScanThreads) k_scan(Ctx c, int initial) {
   if (initial ? c.ctrl->done != 0 : c.ctrl->sort_active == 0) return;
   if (c.ctrl->status & 0x8u) return;
@@ -399,7 +402,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(Ctx c, int initial) {
   for (int k = 0; k < kScanPer; ++k) {
     v[k] = (base + k < c.total_tiles) ? c.s.count[base + k] : 0u;
     sum.x += v[k];
-    sum.y += v[k] > 0u ? 1u : 0u;
+    sum.y += tile_items(v[k], c.split_shift);
   }
   // block exclusive scan of per-thread sums
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -420,7 +423,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(Ctx c, int initial) {
       c.s.rank[base + k] = run.y;
     }
     run.x += v[k];
-    run.y += v[k] > 0u ? 1u : 0u;
+    run.y += tile_items(v[k], c.split_shift);
   }
   if (threadIdx.x == kScanThreads - 1) {  // block totals
     c.s.block_off[blockIdx.x] = run.x;
@@ -461,7 +464,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(Ctx c, int initial) {
   }
   if (threadIdx.x == 0) {
     const unsigned list = c.ctrl->sort_list ^ 1u;
-    c.ctrl->work_count[list] = carry.y;  // non-empty tiles
+    c.ctrl->work_count[list] = carry.y;
     c.ctrl->sort_list = list;
     c.ctrl->in_place = 0u;
     c.ctrl->scan_ticket = 0;
@@ -477,32 +480,32 @@ __device__ __forceinline__ unsigned tile_start(const Ctx& c, unsigned k) {
   return c.s.start[k] + c.s.block_off[k / kScanChunk];
 }
 
-// The same scan by one CTA, 4,096 tiles a round, after a scatter pass that wrote keys (grids of at most
+// The same scan by one CTA, PER tiles a thread and round, after a scatter pass that wrote keys (grids of at most
 // kOpenScanTiles tiles): with most passes keeping their lists it runs once in tens of substeps, where a launch of its own
 // would cost every substep. start and rank come out global here, the block offsets zero.
+template <int PER>
 __device__ __forceinline__ void scan_tiles(const Ctx& c) {
   __shared__ uint2 sums[kScanThreads / 32];
-  constexpr int kPer = kScanPer;
-  const int T = c.total_tiles + 1, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int T = c.total_tiles, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   uint2 carry = make_uint2(0u, 0u);
-  for (int r0 = 0; r0 < T; r0 += kScanThreads * kPer) {
-    const int base = r0 + threadIdx.x * kPer;
-    unsigned v[kPer];
+  for (int r0 = 0; r0 < T; r0 += kScanThreads * PER) {
+    const int base = r0 + threadIdx.x * PER;
+    unsigned v[PER];
     uint2 sum = make_uint2(0u, 0u);
 #pragma unroll
-    for (int q = 0; q < kPer; q += 4) {
-      if (base + q + 4 <= c.total_tiles) {
+    for (int q = 0; q < PER; q += 4) {
+      if (base + q + 4 <= T) {
         const uint4 x = *reinterpret_cast<const uint4*>(c.s.count + base + q);
         v[q] = x.x; v[q + 1] = x.y; v[q + 2] = x.z; v[q + 3] = x.w;
       } else {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) v[q + e] = base + q + e < c.total_tiles ? c.s.count[base + q + e] : 0u;
+        for (int e = 0; e < 4; ++e) v[q + e] = base + q + e < T ? c.s.count[base + q + e] : 0u;
       }
     }
 #pragma unroll
-    for (int q = 0; q < kPer; ++q) {
+    for (int q = 0; q < PER; ++q) {
       sum.x += v[q];
-      sum.y += v[q] > 0u ? 1u : 0u;
+      sum.y += tile_items(v[q], c.split_shift);
     }
     const uint2 incl = warp_incl_scan2(sum, lane);
     __syncthreads();  // sums of the round before are read
@@ -519,14 +522,14 @@ __device__ __forceinline__ void scan_tiles(const Ctx& c) {
       carry.y += x.y;
     }
 #pragma unroll
-    for (int q = 0; q < kPer; q += 4) {
+    for (int q = 0; q < PER; q += 4) {
       unsigned st[4], rk[4];
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         st[e] = run.x;
         rk[e] = run.y;
         run.x += v[q + e];
-        run.y += v[q + e] > 0u ? 1u : 0u;
+        run.y += tile_items(v[q + e], c.split_shift);
       }
       if (base + q + 4 <= T) {
         *reinterpret_cast<uint4*>(c.s.start + base + q) = make_uint4(st[0], st[1], st[2], st[3]);
@@ -541,10 +544,12 @@ __device__ __forceinline__ void scan_tiles(const Ctx& c) {
       }
     }
   }
-  for (int b = threadIdx.x; b * kScanChunk < T; b += kScanThreads) c.s.block_off[b] = c.s.block_rank[b] = 0u;
+  for (int b = threadIdx.x; b * kScanChunk <= T; b += kScanThreads) c.s.block_off[b] = c.s.block_rank[b] = 0u;
   if (threadIdx.x == 0) {
+    c.s.start[T] = carry.x;
+    c.s.rank[T] = carry.y;
     const unsigned list = c.ctrl->sort_list ^ 1u;
-    c.ctrl->work_count[list] = carry.y;  // non-empty tiles
+    c.ctrl->work_count[list] = carry.y;
     c.ctrl->sort_list = list;
     c.ctrl->in_place = 0u;
   }
@@ -553,7 +558,12 @@ __device__ __forceinline__ void scan_tiles(const Ctx& c) {
 // Between two particle passes. scan: a scatter pass came before, and if it wrote keys its counts are
 // scanned; begin: opens the next substep.
 __global__ void __launch_bounds__(kScanThreads) k_open(Ctx c, int begin, int scan) {
-  if (scan && c.ctrl->sort_active != 0 && !(c.ctrl->status & 0x8u)) scan_tiles(c);
+  if (scan && c.ctrl->sort_active != 0 && !(c.ctrl->status & 0x8u)) {
+    if (c.total_tiles <= kScanChunk)
+      scan_tiles<kScanPer>(c);
+    else
+      scan_tiles<16>(c);
+  }
   __syncthreads();
   if (begin) begin_substep(c);
 }
@@ -592,7 +602,9 @@ __device__ __forceinline__ void sort_scatter(const Ctx& c, long long block) {
     const unsigned list = c.ctrl->sort_list;
     const unsigned idx = c.s.rank[key] + c.s.block_rank[key / kScanChunk];
     const int s = c.nscenes == 1 ? 0 : find_scene_by_tile(c.scenes, c.nscenes, static_cast<int>(key));
-    if (idx < static_cast<unsigned>(c.total_tiles)) c.s.work[list][idx] = make_uint4(key, s0, cnt, static_cast<unsigned>(s));
+    const unsigned items = tile_items(cnt, c.split_shift), per = (cnt + items - 1u) / items;
+    for (unsigned q = 0; q < items; ++q)
+      if (idx + q < c.s.work_cap) c.s.work[list][idx + q] = make_uint4(key, s0 + q * per, min(per, cnt - q * per), static_cast<unsigned>(s));
   }
 }
 
@@ -2701,9 +2713,12 @@ __global__ void __launch_bounds__(256) k_cell_order(Ctx c) {
   __shared__ unsigned char cell[kCellSortMax];
   __shared__ int cursor[64];
   const unsigned list = c.ctrl->sort_list;
-  const unsigned nwork = min(c.ctrl->work_count[list], static_cast<unsigned>(c.total_tiles));
+  const unsigned nwork = min(c.ctrl->work_count[list], c.s.work_cap);
   for (unsigned w = blockIdx.x; w < nwork; w += gridDim.x) {
-    const uint4 it = c.s.work[list][w];  // (tile, start, count, scene)
+    uint4 it = c.s.work[list][w];  // (tile, start, count, scene)
+    const unsigned s0 = tile_start(c, it.x);
+    if (it.y != s0) continue;  // a tile's first item stands for the whole tile
+    it.z = tile_start(c, it.x + 1) - s0;
     if (it.z > static_cast<unsigned>(kCellSortMax) || it.y + it.z > static_cast<unsigned long long>(c.n)) continue;
     const SceneDev& sc = c.scenes[it.w];
     if (threadIdx.x < 64) cursor[threadIdx.x] = 0;

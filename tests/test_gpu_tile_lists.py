@@ -1,0 +1,149 @@
+"""Edges of the particle pass's tiles, lists and windows, of the pair search's cells and of the 2D frame
+launch, against the FP64 oracles (GPU tests, through the C ABI).
+
+Tolerances: the device sums FP32 terms, at most N per node. N terms added in any order lie within
+N 2^-24 of the exact sum of their magnitudes, and within about sqrt(N) 2^-24 when roundings are independent;
+four times that, plus the 1e-6 of a few-particle node used elsewhere, bounds the grid normwise. Positions keep the
+1e-6 m of the other step tests, F their 2e-6.
+"""
+import math
+
+import numpy as np
+import pytest
+
+from oracle import oracle as orc
+from oracle.oracle2d import Oracle2
+from mpm_b200 import scenes
+from mpm_b200.params import Domain, Material
+from mpm_b200.solver import Solver
+
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    a, b = np.asarray(a, dtype=np.float64), np.asarray(b, dtype=np.float64)
+    return float(np.max(np.abs(a - b)) / max(np.max(np.abs(b)), 1e-300))
+
+
+def cloud(n, cells, model=0, seed=3):
+    """n particles at random in a cube of `cells` cells that starts on a tile edge of a 16-cell grid."""
+    d = scenes.Domain(lower=(0, 0, 0), upper=(1, 1, 1), H=1 / 16, gravity=(0, -9.8, 0), sticky_floor=True)
+    rng = np.random.default_rng(seed)
+    lo = 4.0 / 16  # node 6 of the grid: base cells from 5.5 on span several tiles
+    x = scenes.quantize_positions(lo + rng.uniform(0, cells / 16, (n, 3)), d)
+    mat = Material.reference_units(model, E=1e5, density=1000.0) if model in (2, 3) else Material.from_young(model, 1e5, .3)
+    sc = scenes._scene("cloud", d, [mat], x, (0, 0, 0))
+    sc.m[:] = 1000.0 * (cells / 16) ** 3 / n
+    sc.V[:] = (cells / 16) ** 3 / n
+    sc.v = np.stack([np.sin(7 * x[:, 1]), np.cos(5 * x[:, 2]), np.sin(6 * x[:, 0])], axis=1)
+    return sc
+
+
+# one particle; a warp, a round of phase A and a scatter round (592), each with one more or less; several
+# rounds per tile; 80,000: more than fit the resident CTAs in parts, so whole tiles of about 2,900
+@pytest.mark.parametrize("n,cells,model", [(1, 1, 0), (31, 1, 0), (33, 2, 0), (255, 2, 0), (257, 2, 0), (591, 2, 0), (593, 2, 0),
+                                           (1300, 2, 0), (2500, 5, 3), (80000, 12, 0)])
+def test_tile_counts(n, cells, model):
+    sc = cloud(n, cells, model)
+    dt = 1e-4
+    sol = Solver(sc.domain, n)
+    sol.upload(sc)
+    st = orc.state_from_scene(sc)
+    gm_ref, gp_ref, _ = st.step(dt, want_grid=True)
+    tol = 1e-6 + 4 * math.sqrt(27 * n / cells ** 3) * 2.0 ** -24
+    gm, gp = sol.grid_debug(dt)
+    assert rel(gm, gm_ref) <= tol
+    assert rel(gp, gp_ref) <= tol
+    sol.step_fixed(dt, 4)
+    for _ in range(3):
+        st.step(dt)
+    out = sol.download(("x", "F"))
+    assert np.max(np.abs(out["x"] - st.x)) <= 1e-6
+    assert np.max(np.abs(out["F"] - st.F)) <= 2e-6
+    assert sol.status() == 0
+    sol.close()
+
+
+# cells travelled per substep: lists kept for the whole run, sorted now and then, sorted every other substep
+@pytest.mark.parametrize("cells_per_step", [.0004, .02, .3])
+def test_lists_follow_a_moving_body(cells_per_step):
+    d = Domain(lower=(0, 0, 0), upper=(1, 1, 1), H=1 / 32)
+    mat = Material.from_young(0, 1e5, .3, density=1000.0)
+    x = scenes.block_particles(d, (6, 6, 6), (13, 11, 12), 5)
+    dt, steps = 1e-4, 40
+    v = cells_per_step * d.H / dt
+    sc = scenes._scene("moving", d, [mat], x, (v, .7 * v, .4 * v))
+    c = x.mean(axis=0)
+    sc.v = sc.v + .05 * v * np.stack([x[:, 1] - c[1], c[0] - x[:, 0], 0 * x[:, 2]], axis=1) / d.H / 8
+    sol = Solver(sc.domain, sc.n)
+    sol.upload(sc)
+    st = orc.state_from_scene(sc)
+    sol.step_fixed(dt, steps)
+    for _ in range(steps):
+        st.step(dt)
+    out = sol.download(("x", "F"))
+    # a position is rounded to H / 2^22 each substep, and each substep adds dt v with FP32's v
+    tol = 1e-6 + steps * d.H / 2 ** 23 + 4 * steps * dt * v * 2.0 ** -24
+    assert np.max(np.abs(out["x"] - st.x)) <= tol
+    assert np.max(np.abs(out["F"] - st.F)) <= 2e-6 * max(1.0, 40 * cells_per_step)
+    assert sol.status() == 0
+    sol.close()
+
+
+# the fine cells of a filled grid and the coarse ones of a mostly empty grid
+@pytest.mark.parametrize("spacing,radius", [(2.8, 8.0), (.45, .8)])
+def test_pair_cells(spacing, radius):
+    d = Domain(lower=(-64, -48, -64), upper=(64, 72, 64), H=8.0)
+    rng = np.random.default_rng(9)
+    n = 1200
+    x = rng.uniform(-4 * spacing, 4 * spacing, (n, 3))
+    mats = [Material(model=0, mu=.4, lam=.4, specific_heat=cp, conductivity=k) for cp, k in ((4180.0, .6), (450.0, 80.0))]
+    sc = scenes._scene("pairs", d, mats, x, (0, 0, 0))
+    sc.m, sc.V = rng.uniform(.5, 2.0, n), rng.uniform(.5, 1.5, n)
+    sc.mat = (rng.uniform(0, 1, n) < .4).astype(np.int32)
+    sc.T = rng.uniform(20, 300, n)
+    kw = dict(spacing=spacing, volume_unit=1.0, max_speed=8.0, rate=40.0)
+    sol = Solver(d, n)
+    sol.upload(sc)
+    st = orc.state_from_scene(sc)
+    st.init_enthalpy()
+    sol.exchange_heat(1 / 60, radius)
+    st.exchange_heat(1 / 60, radius=radius)
+    assert np.max(np.abs(sol.download(("T",))["T"] - st.T)) <= 1e-4 * 300
+    sol.set_regularizer(True, **kw)
+    sol.regularize(1 / 240)
+    st.regularize(1 / 240, **kw)
+    # one rounding of a position to H / 2^22, and FP32 shifts of at most max_speed dt
+    assert np.max(np.abs(sol.download(("x",))["x"] - st.x)) <= d.H / 2 ** 22 + 8 / 240 * 4e-6
+    sol.close()
+
+
+# one launch for the frame (one particle per resident thread) and, above that, launches per substep
+@pytest.mark.parametrize("nx,ny", [(1, 1), (127, 1), (43, 3), (200, 200)])
+def test_plane_frame_launches(nx, ny):
+    from mpm_b200.solid_mpm import SolidMPM, SolidSim
+    n = nx * ny
+
+    def sim():
+        s = SolidSim(n, gravity="center")
+        g = np.random.default_rng(4)
+        s.count = n
+        s.x[:n] = (np.tile(np.arange(nx), ny) - nx / 2) * 3.6 + g.uniform(-.3, .3, n)
+        s.y[:n] = (np.repeat(np.arange(ny), nx) - ny / 2) * 3.6 + g.uniform(-.3, .3, n)
+        s.vx[:n], s.vy[:n] = g.uniform(-5, 5, n), g.uniform(-5, 5, n)
+        s.mass[:n], s.volume[:n], s.material[:n] = 1.1, 1.0, 11
+        s.pinned[:n] = g.uniform(0, 1, n) < .02
+        s.material[:n][g.uniform(0, 1, n) < .03] = 0  # not a solid: left alone
+        return s
+
+    s, t = sim(), sim()
+    m, o = SolidMPM(n), Oracle2(n)
+    for _ in range(3):
+        ng, ag = m.frame(s)
+        nc, ac = o.frame(t)
+        assert ng == nc and abs(ag - ac) < 1e-9
+    extent = 1192.0
+    assert np.abs(s.x[:n].astype(np.float64) - t.x[:n]).max() <= 1e-5 * extent
+    assert np.abs(s.y[:n].astype(np.float64) - t.y[:n]).max() <= 1e-5 * extent
+    assert m.stats(s)["nodes"] == o.stats(t)["nodes"]
+    m.close()
