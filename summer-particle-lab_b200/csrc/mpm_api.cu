@@ -1441,7 +1441,7 @@ int mpm_regularize(mpm_handle* h, double dt) {
   return MPM_OK;
 }
 
-// Lays out the heat-exchange scratch for cells one radius wide over each scene's grid.
+// Lays out the heat-exchange scratch for cells half a radius (or one, see choose_cells) wide over each scene's grid.
 static int ensure_heat(mpm_handle* h, double radius) {
   if (h->hblock && h->heat_radius == radius) return MPM_OK;
   const int ns = static_cast<int>(h->scenes.size());

@@ -98,7 +98,7 @@ struct Ctrl {
   unsigned strays;       // particles that left the tile whose list holds them, as of the last scatter pass
   unsigned far_strays;   // some of them a whole cell or more
   unsigned in_place;     // perm is the identity: the state was permuted after the newest sort
-  unsigned last_substep; // 1 when the current substep is the call's last (set by k_begin): only then
+  unsigned last_substep; // 1 when the current substep is the call's last (set by k_open): only then
                          // does the fused pass store particle velocities and APIC matrices, which no
                          // later substep of the call reads
 };
