@@ -107,7 +107,8 @@ struct mpm_handle {
   void* rblock = nullptr;  size_t rblock_bytes = 0;
   mpm::RegBufs rbufs{};
   mpm::RegDev rdev{};
-  bool reg_dirty = true;   // domain, scenes or spacing changed since the scratch was laid out
+  bool reg_dirty = true;   // domain or scenes changed since the scratch was laid out
+  double reg_spacing = 0;  // spacing the scratch was laid out for
   // particle-pair heat exchange scratch, laid out for heat_radius
   void* hblock = nullptr;  size_t hblock_bytes = 0;
   mpm::HeatBufs hbufs{};
@@ -1104,8 +1105,7 @@ static long long choose_cells(const mpm_handle* h, double fine, double coarse, s
 
 // Lays out the regularisation scratch for the current scenes and spacing: neighbour cells one spacing
 // (or two, see choose_cells) wide over each scene's grid, the cell sort and the per-particle shifts.
-static int ensure_regularizer(mpm_handle* h) {
-  if (!h->reg_dirty && h->rblock) return MPM_OK;
+static int lay_out_regularizer(mpm_handle* h) {
   const int ns = static_cast<int>(h->scenes.size());
   std::vector<mpm::RegScene> rs;
   double hc = 0;
@@ -1148,14 +1148,25 @@ static int ensure_regularizer(mpm_handle* h) {
   mpm::RegDev& r = h->rdev;
   r.scenes = sp;
   r.cells = cells;
+  r.hc = static_cast<float>(hc);
+  r.inv_hc = static_cast<float>(1.0 / hc);
+  h->reg_dirty = false;
+  h->reg_spacing = h->reg.spacing;
+  return MPM_OK;
+}
+
+// The scratch for the current scenes and spacing, and the current parameters.
+static int ensure_regularizer(mpm_handle* h) {
+  if (h->reg_dirty || !h->rblock || h->reg_spacing != h->reg.spacing) {
+    const int rc = lay_out_regularizer(h);
+    if (rc != MPM_OK) return rc;
+  }
+  mpm::RegDev& r = h->rdev;
   r.spacing = static_cast<float>(h->reg.spacing);
   r.inv_volume_unit = static_cast<float>(1.0 / h->reg.volume_unit);
   r.max_speed = static_cast<float>(h->reg.max_speed);
   r.rate = static_cast<float>(h->reg.rate);
   r.eps = static_cast<float>(h->reg.spacing * 1e-8 / 2.8);  // 1e-8 in the reference's units (spacing 2.8)
-  r.hc = static_cast<float>(hc);
-  r.inv_hc = static_cast<float>(1.0 / hc);
-  h->reg_dirty = false;
   return MPM_OK;
 }
 
@@ -1424,7 +1435,6 @@ int mpm_set_regularizer(mpm_handle* h, const mpm_regularizer* r) {
                      !std::isfinite(r->spacing) || !std::isfinite(r->volume_unit) || !std::isfinite(r->max_speed) ||
                      !std::isfinite(r->rate)))
     return fail(h, MPM_ERR_INVALID_ARG, "regulariser needs spacing, volume_unit, max_speed > 0 and rate >= 0");
-  if (r->enabled && r->spacing != h->reg.spacing) h->reg_dirty = true;
   h->reg = *r;
   drop_graph(h);  // a captured graph holds the fused (unregularised) substeps
   return MPM_OK;

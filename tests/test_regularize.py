@@ -203,3 +203,27 @@ def test_device_substeps_with_regularisation_match_oracle():
     assert np.max(np.abs(out["F"] - st.F)) <= 1e-6
     assert sol.status() == 0
     sol.close()
+
+
+# each parameter on its own, and a spacing that was set while the pass was off
+@pytest.mark.gpu
+@pytest.mark.parametrize("change", [dict(rate=.05), dict(max_speed=.5), dict(volume_unit=.3), dict(spacing=2.0)])
+@pytest.mark.parametrize("while_off", [False, True])
+def test_device_takes_parameters_changed_after_a_pass(change, while_off):
+    from mpm_b200.solver import Solver
+    kw = dict(spacing=2.8, volume_unit=1.0, max_speed=8.0, rate=40.0)
+    sc = crowded_cloud()
+    st = orc.state_from_scene(sc)
+    sol = Solver(sc.domain, sc.n)
+    sol.upload(sc)
+    sol.set_regularizer(True, **kw)
+    sol.regularize(1 / 240)
+    st.regularize(1 / 240, **kw)
+    kw.update(change)
+    if while_off:
+        sol.set_regularizer(False, **kw)
+    sol.set_regularizer(True, **kw)
+    sol.regularize(1 / 240)
+    st.regularize(1 / 240, **kw)
+    assert np.max(np.abs(sol.download(("x",))["x"] - st.x)) <= 2 * 1e-6 * 2.8  # two passes of the cloud test's bound
+    sol.close()
