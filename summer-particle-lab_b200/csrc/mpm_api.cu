@@ -1514,6 +1514,9 @@ int mpm_exchange_heat(mpm_handle* h, const mpm_heat_exchange* x, double dt, doub
   if (rc != MPM_OK) return rc;
   mpm::HeatDev hd = h->hdev;
   hd.radius = static_cast<float>(x->radius);
+  const double inv_radius = 1.0 / static_cast<double>(hd.radius);
+  hd.inv_radius = static_cast<float>(inv_radius);
+  hd.inv_radius_lo = static_cast<float>(inv_radius - static_cast<double>(hd.inv_radius));
   hd.eps = static_cast<float>(x->radius * 1.25e-7);  // 1e-6 of the reference's 8-unit radius
   hd.geom_rate = static_cast<float>(x->geometry * x->heat_rate);
   hd.dt = static_cast<float>(dt);

@@ -64,13 +64,6 @@ __device__ __forceinline__ void ball_rows(const RegScene& rs, const unsigned* st
   }
 }
 
-// Square root to 2^-23 relative (one instruction; the rounded one took 5% of the heat passes).
-__device__ __forceinline__ float sqrt_approx(float x) {
-  float r;
-  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-
 __global__ void k_reg_count(Ctx c, RegDev r, unsigned* cell_of, float* target, float* inv_mass, unsigned* count,
                             unsigned* tmax) {
   for (long long h = blockIdx.x * (long long)blockDim.x + threadIdx.x; h < c.n; h += (long long)gridDim.x * blockDim.x) {
@@ -325,7 +318,7 @@ __device__ __forceinline__ void heat_pairs(const Ctx& c, const HeatDev& hd, cons
   const uint4 pi = pos_sorted[ks];
   const float ki = prop_sorted[ks].x;
   const float to_m = sc.H * kInvFixedOne;
-  const float inv_radius = 1.f / hd.radius, r2_max = hd.radius * hd.radius * 1.000001f;
+  const float r2_max = hd.radius * hd.radius * 1.000001f;
   const float xi[3] = {static_cast<float>(pi.x) * kInvFixedOne * sc.H, static_cast<float>(pi.y) * kInvFixedOne * sc.H,
                        static_cast<float>(pi.z) * kInvFixedOne * sc.H};
   ball_rows(hd.scenes[s], start, xi, hd.radius, hd.hc, hd.inv_hc, [&](unsigned b, unsigned e) {
@@ -337,18 +330,23 @@ __device__ __forceinline__ void heat_pairs(const Ctx& c, const HeatDev& hd, cons
       const float dz = static_cast<float>(static_cast<int>(pi.z - pj.z)) * to_m;
       const float r2 = dx * dx + dy * dy + dz * dz;
       if (r2 > r2_max) continue;
-      const float r = sqrt_approx(r2);
+      const float r = sqrtf(r2);
       if (!(r > hd.eps && r < hd.radius) || k == ks) continue;
       const float kj = prop_sorted[k].x;
       // no division inside one material
       const float kh = ki == kj ? ki : ki + kj > 0.f ? 2.f * ki * kj / (ki + kj) : 0.f;
-      fn(k, (1.f - r * inv_radius) * hd.geom_rate * kh);
+      // 1 - r / radius by the reciprocal's two parts, each product unrounded: the weight keeps its digits
+      // where it goes to zero
+      const float weight = fmaf(-r, hd.inv_radius_lo, fmaf(-r, hd.inv_radius, 1.f));
+      fn(k, weight * hd.geom_rate * kh);
     }
   });
 }
 
 // 128-thread CTAs at 48 registers: the search is a chain of cached loads, and 40 resident warps per SM hide
-// them better than 32 at 64 registers (768 us for both passes at 357,120 particles, 832 there; 796 at 48 warps, 850 at 64).
+// them better than 36 or 32, though at 48 registers 24 bytes spill. Exchange at 357,120 particles 749 us (780,
+// 855), at 195,776 474 (529, 560); where the particles no longer fill those warps it is the spills that show: at
+// 131,376 351 (336, 330), at 39,600 303 (290, 289).
 constexpr int kHeatThreads = 128;
 
 __global__ void __launch_bounds__(kHeatThreads, 10) k_heat_budget(Ctx c, HeatDev hd, const unsigned* start, const unsigned* sorted, const uint4* pos_sorted, const float2* prop_sorted, float* budget) {

@@ -48,6 +48,7 @@ struct HeatDev {
   long long cells;
   float hc, inv_hc;     // neighbour cell size (see ensure_heat) and its inverse
   float radius, eps;    // pairs with eps < r < radius
+  float inv_radius, inv_radius_lo;  // 1 / radius in two parts
   float geom_rate;      // geometry * heat_rate
   float dt;
   int ambient;

@@ -208,3 +208,29 @@ def test_device_cloud_matches_oracle():
     e = float(np.sum(sc.m * out["enthalpy"]))
     assert abs(e - before) <= 1e-6 * abs(before)
     assert abs(q - qo) <= 1e-4 * qo
+
+
+# the pair weight 1 - r / radius to FP32 rounding from r = radius / 64 to 127 / 128 of the radius: isolated pairs
+# along x, whose distances are exact in FP32, as are their squares and the roots of those
+@pytest.mark.gpu
+@pytest.mark.parametrize("radius", [8.0, 7.0, 5.125, .8])
+def test_device_pair_weight_keeps_its_digits(radius):
+    radius = float(np.float32(radius))
+    unit = DOMAIN.H / 2 ** 10
+    steps = np.unique(np.round(np.concatenate([np.arange(1, 64) / 64, [127 / 128]]) * radius / unit).astype(int))
+    dist = steps[steps * unit < radius] * unit
+    y, z = np.meshgrid(np.arange(-40, 64, 11), np.arange(-60, 60, 11), indexing="ij")
+    rows = np.stack([y.ravel(), z.ravel()], axis=1)[:len(dist)]
+    assert len(rows) == len(dist)
+    left = np.column_stack([np.full(len(dist), -16.0), rows])
+    right = left + np.column_stack([dist, np.zeros_like(rows)])
+    sc = heat_scene(np.concatenate([left, right]), [0.0] * len(dist) + [512.0] * len(dist), [IRON] * (2 * len(dist)))
+    dt, heat_rate = 2.0 ** -10, 20.0
+    out, _ = device(sc, 1, dt, radius, heat_rate)
+    # FP32 inputs, 64-bit arithmetic: the temperature gained from 0 by the left particle of each pair
+    f = lambda v: float(np.float32(v))
+    k, m, cp = f(IRON["k"]), f(IRON["m"]), f(IRON["cp"])
+    gain = 512.0 * (1 - dist / radius) * f(20.0 * heat_rate) * k * dt / (m * cp)
+    assert np.all(gain < .2 * 512)  # no budget cuts in
+    # two sums of the weight, geometry, conductivity, stored temperature: a rounding each
+    assert np.max(np.abs(out["T"][:len(dist)] / gain - 1)) <= 5 * 2.0 ** -24
