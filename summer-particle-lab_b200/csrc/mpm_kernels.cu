@@ -158,13 +158,6 @@ __device__ __forceinline__ double warp_sum_d(double x) {
 
 __device__ __forceinline__ unsigned fbits(float x) { return __float_as_uint(fmaxf(x, 0.f)); }
 
-// Square root for the CFL terms: x rsqrt(x), two units in the last place at most; arguments outside
-// [1e-30, 3e38] are moved to the ends of that range.
-__device__ __forceinline__ float sqrt_bounded(float x) {
-  const float y = fminf(fmaxf(x, 1e-30f), 3e38f);
-  return y * rsqrtf(y);
-}
-
 // CFL terms of src/three/mpm.js:43-54 for one particle (F = I + D)
 template <bool AUX>
 __device__ __forceinline__ void cfl_terms(const MaterialDev& mt, const float D[9], const float v[3],
@@ -187,8 +180,8 @@ __device__ __forceinline__ void cfl_terms(const MaterialDev& mt, const float D[9
   // moduli carry its hardening
   const bool press = AUX && (mt.model == 8 || mt.model == 9);
   const float compression = mt.model == 1 || press ? 1.f / fmaxf(0.05f, (1.f + Jm1) * (press ? 1.f + aux : 1.f)) : 1.f;
-  const float c = sqrt_bounded(mt.wave_modulus * (AUX && mt.model == 2 ? snow_hardening(aux) : 1.f) * (V / m));
-  const float speed = sqrt_bounded(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+  const float c = sqrtf(mt.wave_modulus * (AUX && mt.model == 2 ? snow_hardening(aux) : 1.f) * V / m);
+  const float speed = sqrtf(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
   wave = speed + c * fmaxf(1.f, fmaxf(row * col, compression));
   grad = g;
 }

@@ -386,3 +386,21 @@ def test_johnson_cook_on_dense_tiles_matches_oracle():
     assert np.max(np.abs(out["ep"] - st.ep)) <= 2e-6 + 1e-4 * np.max(st.ep)
     assert sol.status() == 0
     sol.close()
+
+
+def test_stable_dt_takes_rounded_roots():
+    """The CFL terms c = sqrt(M V / m) and |v| of particles whose squares, products and quotients are exact
+    in FP32: the step follows from correctly rounded roots to the last bit (src/three/mpm.js:43-54)."""
+    d = scenes.Domain(lower=(0, 0, 0), upper=(1, 1, 1), H=1 / 16, cfl=.5)
+    one = scenes._scene("one", d, [Material(model=0, mu=1.0, lam=1.0)], np.array([[.5, .5, .5]]), (0, 0, 0))
+    sol = Solver(d, 1)
+    # wave speeds from 3 to 4093 m/s at rest, then |v| from 3 to 3021 m/s (1, 2, 2 and 2, 3, 6) beside c = 2 m/s
+    states = [(c, (0, 0, 0), c) for c in range(3, 4096, 10)]
+    states += [(2, (k, 2 * k, 2 * k), 3 * k + 2) for k in range(1, 1000, 14)] + [(2, (6 * k, 3 * k, 2 * k), 7 * k + 2) for k in range(1, 430, 9)]
+    for c, v, wave in states:
+        mu = 1024.0 * c * c / 4
+        one.materials = [Material(model=0, mu=mu, lam=2 * mu)]
+        one.m, one.V, one.v = np.array([1024.0]), np.array([1.0]), np.array([v], dtype=np.float64)
+        sol.upload(one)
+        assert np.float32(sol.stable_dt()) == np.float32(d.cfl * d.H) / np.float32(wave), (c, v)
+    sol.close()
