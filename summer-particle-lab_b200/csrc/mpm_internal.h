@@ -97,6 +97,7 @@ struct Ctrl {
   unsigned sort_want;    // 1: the next scatter pass writes keys (set by the substep's prologue from the two below)
   unsigned strays;       // particles that left the tile whose list holds them, as of the last scatter pass
   unsigned far_strays;   // some of them a whole cell or more
+  unsigned list_age;     // substeps since the state was last sorted (0: every particle is listed in its own tile)
   unsigned in_place;     // perm is the identity: the state was permuted after the newest sort
   unsigned last_substep; // 1 when the current substep is the call's last (set by k_open): only then
                          // does the fused pass store particle velocities and APIC matrices, which no

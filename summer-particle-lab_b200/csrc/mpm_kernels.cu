@@ -207,6 +207,7 @@ __global__ void k_control(Ctx c, ControlOp op) {
     ct->last_substep = 1u;
     if (op.op == 0) {
       ct->sort_active = ct->sort_want = ct->strays = ct->far_strays = 0u;
+      ct->list_age = 0xffffffffu;  // 0 in the first substep
       ct->active_count[k & 1] = 0;
       ct->work_next = 0;
       ct->done = 0;
@@ -315,6 +316,7 @@ __device__ __forceinline__ void begin_substep(const Ctx& c) {
       // and to the tile's window (at 1 in 32 a full tile has about 20 more non-empty buckets than 64). A particle
       // a whole cell out is one cell from leaving the windows, so it asks for a sort at once.
       ct->sort_want = !ct->sort_active && (ct->far_strays != 0u || ct->strays > c.n / kStrayShare) ? 1u : 0u;
+      ct->list_age = ct->sort_active ? 0u : ct->list_age + 1u;
       ct->strays = 0u;
       ct->far_strays = 0u;
     }
@@ -1064,6 +1066,28 @@ __device__ __noinline__ Gather12 gather_global(const float4* base, int sy, long 
   return g;
 }
 
+// Whether a move from q0 to q1 along one axis takes a stencil out of the scatter window of the tile that q0 lies in.
+__device__ __forceinline__ bool leaves_tile_window(unsigned q0, unsigned q1, int dim) {
+  int b0, b1;
+  float t;
+  stencil_axis(q0, dim, b0, t);
+  stencil_axis(q1, dim, b1, t);
+  const int l = b1 - (b0 & ~(kTile - 1)) + 1;
+  return l < 0 || l > kWinS - 3;
+}
+
+// MPM_STATUS_SCATTER_OVERFLOW for a particle about to be stored at q: a move of more than a cell out of the scatter
+// window of the tile it came from, whichever tile's list holds it. Position and velocity are what a caller has at
+// hand; the old position is read back from the state only in the branch (kept in registers it cost the
+// pass 2%, this 0.6%: 276.2 -> 278.2 us at 2,097,152 particles). A particle that the box moved further than its velocity has a list of age 0.
+__device__ __forceinline__ void report_long_move(const Ctx& c, const TileCtx& tc, unsigned home, const unsigned q[3],
+                                                 const float v[3], float dt) {
+  if (fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fabsf(v[2])) * (dt * tc.invH) < 0.999f) return;
+  if (leaves_tile_window(c.p.qx[home], q[0], tc.dims[0]) || leaves_tile_window(c.p.qy[home], q[1], tc.dims[1]) ||
+      leaves_tile_window(c.p.qz[home], q[2], tc.dims[2]))
+    atomicOr(&c.ctrl->status, 0x10u);
+}
+
 // A stray (window bases 1..4 are the tile's, 0 and 5 one cell out) within a quarter cell of leaving the
 // windows.
 __device__ __forceinline__ bool near_window_end(int l0, float t0, int l1, float t1, int l2, float t2) {
@@ -1210,9 +1234,10 @@ __device__ __forceinline__ unsigned particle_phase_a(const Ctx& c, const SceneDe
     }
     ep += co.dep;
     T += co.dT;
-    c.p.qx[home] = q[0]; c.p.qy[home] = q[1]; c.p.qz[home] = q[2];
 #pragma unroll
     for (int e = 0; e < 9; ++e) c.p.Dc[e][home] = D[e];
+    if (SCATTER) report_long_move(c, tc, home, q, v, dt);
+    c.p.qx[home] = q[0]; c.p.qy[home] = q[1]; c.p.qz[home] = q[2];
     // v and C: the fused pass scatters the ones it just gathered and never reads the stored copies,
     // so it stores them only on the call's last substep (downloads, ledgers, frames, regularisation
     // and a later P2G of the stored state read them after the call); the gather-only pass always does
@@ -1279,8 +1304,7 @@ __device__ __forceinline__ unsigned particle_phase_a(const Ctx& c, const SceneDe
       if (!in_w) {
         stray = true;
         flags |= kFlagFar;
-        const float cells = dt * tc.invH;  // more than a cell in this substep
-        if (fabsf(cells * v[0]) > 1.f || fabsf(cells * v[1]) > 1.f || fabsf(cells * v[2]) > 1.f) flags |= 0x10u;
+        if (c.ctrl->list_age == 0u) flags |= 0x10u;  // the window is that of the particle's own tile
       }
       // copies scoped to this rare branch: the arrays passed to the out-of-line scatter would
       // otherwise live in local memory on every particle's path (3% of the fused pass)
@@ -1451,6 +1475,7 @@ __device__ __forceinline__ unsigned particle_phase_a_learned(const Ctx& c, const
     ep += co.dep;
     T += co.dT;
     if (live) {
+      if (SCATTER) report_long_move(c, tc, home, q, v, dt);
       c.p.qx[home] = q[0]; c.p.qy[home] = q[1]; c.p.qz[home] = q[2];
 #pragma unroll
       for (int e = 0; e < 9; ++e) c.p.Dc[e][home] = D[e];
@@ -1511,8 +1536,7 @@ __device__ __forceinline__ unsigned particle_phase_a_learned(const Ctx& c, const
       if (!in_w) {
         stray = true;
         flags |= kFlagFar;
-        const float cells = dt * tc.invH;  // more than a cell in this substep
-        if (fabsf(cells * v[0]) > 1.f || fabsf(cells * v[1]) > 1.f || fabsf(cells * v[2]) > 1.f) flags |= 0x10u;
+        if (c.ctrl->list_age == 0u) flags |= 0x10u;  // the window is that of the particle's own tile
       }
       // copies scoped to this rare branch: the arrays passed to the out-of-line scatter would
       // otherwise live in local memory on every particle's path

@@ -147,3 +147,36 @@ def test_plane_frame_launches(nx, ny):
     assert np.abs(s.y[:n].astype(np.float64) - t.y[:n]).max() <= 1e-5 * extent
     assert m.stats(s)["nodes"] == o.stats(t)["nodes"]
     m.close()
+
+
+# MPM_STATUS_SCATTER_OVERFLOW (0x10) follows from a particle's own tile before and after a move, not from the tile whose
+# list holds it. One flyer beside 64 pinned particles (so one stray in 65 keeps the lists); start in cells from the
+# grid's origin, velocity in cells, acceleration, substep lengths. In turn: out of a kept list's tile by the near
+# side and back across both its sides; out by the far side and on inside the next tile; moves of more than a cell in fresh
+# lists that leave the window and that do not; from outside the box into it
+@pytest.mark.parametrize("x0,cells,gravity,dts", [(4.51, -.02, True, (1e-4, 1e-2)), (8.49, .02, False, (1e-4, 65e-4)), (7.2, 1.5, False, (1e-4,)),
+                                                  (4.6, 2.3, False, (1e-4,)), (7.2, -1.3, False, (1e-4,)), (19.9, -.01, False, (1e-4, 1e-4)),
+                                                  (.2, .01, False, (1e-4, 1e-4))])
+def test_overflow_status_follows_a_particles_own_tile(x0, cells, gravity, dts):
+    h = 1 / 16
+    v = cells * h / dts[0]
+    g = (1.3 * h / dts[1] - v) / (dts[0] + dts[1]) if gravity else 0.0
+    d = Domain(lower=(0, 0, 0), upper=(1, 1, 1), H=h, gravity=(g, 0, 0))
+    o = np.asarray(d.origin)
+    grid = np.stack(np.meshgrid(*[13.25 + .5 * np.arange(4)] * 3), axis=-1).reshape(-1, 3)
+    x = scenes.quantize_positions(o + h * np.concatenate([[[x0, 6.3, 6.3]], grid]), d)
+    sc = scenes._scene("flyer", d, [Material.from_young(0, 1e5, .3, density=1000.0)], x, (0, 0, 0))
+    sc.v[0, 0] = v
+    sc.pinned = (np.arange(len(x)) > 0).astype(np.uint8)
+    sol = Solver(d, len(x))
+    sol.upload(sc)
+    base = lambda p: np.clip(np.floor((p - o) / h - .5), 0, np.asarray(d.dims) - 3).astype(int)
+    before, expected = base(x[0]), 0
+    for dt in dts:
+        sol.step_fixed(dt, 1)
+        after = base(sol.download(("x",))["x"][0])
+        local = after - (before // 4 * 4 - 1)
+        expected |= 0x10 if np.any((local < 0) | (local > 5)) else 0
+        assert sol.status() == expected, (before, after)
+        before = after
+    sol.close()
