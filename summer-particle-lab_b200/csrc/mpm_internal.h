@@ -94,9 +94,10 @@ struct Ctrl {
   int step_substeps;     // substeps of the current requested-dt step
   unsigned sort_list;    // the newest work list: what a particle pass reads, and the sort after a scan writes
   unsigned sort_active;  // 1 if the last scatter pass wrote keys to sort (the scan and sort do nothing otherwise)
-  unsigned sort_want;    // 1: the next scatter pass writes keys (set by the substep's prologue from the two below)
+  unsigned sort_want;    // 1: the next scatter pass writes keys (set by the substep's prologue from the three below)
   unsigned strays;       // particles that left the tile whose list holds them, as of the last scatter pass
-  unsigned far_strays;   // some of them a whole cell or more
+  unsigned far_strays;   // some of them may leave the windows next (kFlagFar), moving fast (kFlagFast)
+  unsigned first_speed;  // the largest particle speed, in cells per second (float bits), of a P2G pass's state
   unsigned list_age;     // substeps since the state was last sorted (0: every particle is listed in its own tile)
   unsigned in_place;     // perm is the identity: the state was permuted after the newest sort
   unsigned last_substep; // 1 when the current substep is the call's last (set by k_open): only then

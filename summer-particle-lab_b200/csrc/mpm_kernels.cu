@@ -190,6 +190,9 @@ __device__ __forceinline__ void cfl_terms(const MaterialDev& mt, const float D[9
 // control
 
 constexpr unsigned kStrayShare = 32;
+// In a pass's status word, beside MPM_STATUS_*: a stray that the next substep may take out of the windows, and one
+// that moves more than half a cell in a substep.
+constexpr unsigned kFlagFar = 0x80000000u, kFlagFast = 0x40000000u;
 
 struct ControlOp {
   int op;           // 0: reset lists for an initial sort + P2G, 1: start a step call
@@ -206,7 +209,7 @@ __global__ void k_control(Ctx c, ControlOp op) {
     const unsigned k = ct->step_index;
     ct->last_substep = 1u;
     if (op.op == 0) {
-      ct->sort_active = ct->sort_want = ct->strays = ct->far_strays = 0u;
+      ct->sort_active = ct->sort_want = ct->strays = ct->far_strays = ct->first_speed = 0u;
       ct->list_age = 0xffffffffu;  // 0 in the first substep
       ct->active_count[k & 1] = 0;
       ct->work_next = 0;
@@ -314,8 +317,13 @@ __device__ __forceinline__ void begin_substep(const Ctx& c) {
       ct->grid_next = 0;
       // Sort again when one particle in kStrayShare has left its tile: strays add to the buckets of phase B
       // and to the tile's window (at 1 in 32 a full tile has about 20 more non-empty buckets than 64). A particle
-      // a whole cell out is one cell from leaving the windows, so it asks for a sort at once.
-      ct->sort_want = !ct->sort_active && (ct->far_strays != 0u || ct->strays > c.n / kStrayShare) ? 1u : 0u;
+      // that may leave the windows asks for a sort at once. Past half a cell a substep, two substeps with one list
+      // outrun the windows and what is out of them is scattered in global memory (2,097,152 particles at .9 cells:
+      // 1770 us a substep, 425 sorted every time), so every pass writes keys, the first one by the speeds of the
+      // state that was scattered.
+      const bool fast = (ct->far_strays & kFlagFast) != 0u || dt * __uint_as_float(ct->first_speed) > 0.5f;
+      ct->sort_want = fast || (!ct->sort_active && (ct->far_strays != 0u || ct->strays > c.n / kStrayShare)) ? 1u : 0u;
+      ct->first_speed = 0u;
       ct->list_age = ct->sort_active ? 0u : ct->list_age + 1u;
       ct->strays = 0u;
       ct->far_strays = 0u;
@@ -649,7 +657,6 @@ constexpr int kBuckets = 216;  // 6^3 possible stencil bases in the scatter wind
 __device__ __forceinline__ int pay_slot(int j) { return j ^ ((j >> 3) & 7); }
 static_assert(kCap % 8 == 0, "pay_slot permutes within blocks of eight");
 constexpr unsigned kMetaInvalid = 0x80000000u;
-constexpr unsigned kFlagFar = 0x80000000u;  // beside the status flags: a stray a whole cell out of its tile
 
 enum Pass : int { kPassP2G = 0, kPassG2P2G = 1, kPassG2P = 2 };
 
@@ -680,7 +687,7 @@ struct __align__(128) PartSmem {
   unsigned long long mbar;
   uint4 item[2];
   int abort_flag;
-  unsigned red[4];   // the tile's CFL maxima (float bits), status flags (and kFlagFar), strays
+  unsigned red[4];   // the tile's CFL maxima (float bits), status flags (with kFlagFar, kFlagFast), strays (P2G: speed)
   unsigned gate[2];  // learned mode: returns the gate accepted / sent to the bisection
   // State the CTA carries from tile to tile sits here rather than in registers: at 128 registers a
   // thread, every register held across the tiles is one fewer for phase A, and moving these (with
@@ -1076,31 +1083,39 @@ __device__ __forceinline__ bool leaves_tile_window(unsigned q0, unsigned q1, int
   return l < 0 || l > kWinS - 3;
 }
 
-// MPM_STATUS_SCATTER_OVERFLOW for a particle about to be stored at q: a move of more than a cell out of the scatter
-// window of the tile it came from, whichever tile's list holds it. Position and velocity are what a caller has at
-// hand; the old position is read back from the state only in the branch (kept in registers it cost the
-// pass 2%, this 0.6%: 276.2 -> 278.2 us at 2,097,152 particles). A particle that the box moved further than its velocity has a list of age 0.
-__device__ __forceinline__ void report_long_move(const Ctx& c, const TileCtx& tc, unsigned home, const unsigned q[3],
-                                                 const float v[3], float dt) {
-  if (fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fabsf(v[2])) * (dt * tc.invH) < 0.999f) return;
-  if (leaves_tile_window(c.p.qx[home], q[0], tc.dims[0]) || leaves_tile_window(c.p.qy[home], q[1], tc.dims[1]) ||
-      leaves_tile_window(c.p.qz[home], q[2], tc.dims[2]))
-    atomicOr(&c.ctrl->status, 0x10u);
+// The largest move along an axis, in cells, of a substep at velocity v.
+__device__ __forceinline__ float largest_move(const float v[3], float dt, float invH) {
+  return fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fabsf(v[2])) * (dt * invH);
 }
 
-// A stray (window bases 1..4 are the tile's, 0 and 5 one cell out) within a quarter cell of leaving the
-// windows.
-__device__ __forceinline__ bool near_window_end(int l0, float t0, int l1, float t1, int l2, float t2) {
-  return (l0 == 0 && t0 < 0.75f) || (l0 == 5 && t0 > 1.25f) || (l1 == 0 && t1 < 0.75f) || (l1 == 5 && t1 > 1.25f) ||
-         (l2 == 0 && t2 < 0.75f) || (l2 == 5 && t2 > 1.25f);
+// MPM_STATUS_SCATTER_OVERFLOW for a particle about to be stored at q: a move of more than a cell out of the scatter
+// window of the tile it came from, whichever tile's list holds it. Position and velocity are what a caller has at
+// hand; the old position is read back from the state only in the branch (kept in registers it cost the pass 2%, this
+// 0.7%: 276.2 -> 278.2 us at 2,097,152 particles). A particle that the box moved further than its velocity has a list
+// of age 0.
+__device__ __forceinline__ void report_long_move(const Ctx& c, const TileCtx& tc, unsigned home, const unsigned q[3],
+                                                 const float v[3], float dt) {
+  if (largest_move(v, dt, tc.invH) < 0.999f) return;
+  if (leaves_tile_window(c.p.qx[home], q[0], tc.dims[0])) atomicOr(&c.ctrl->status, 0x10u);
+  if (leaves_tile_window(c.p.qy[home], q[1], tc.dims[1])) atomicOr(&c.ctrl->status, 0x10u);
+  if (leaves_tile_window(c.p.qz[home], q[2], tc.dims[2])) atomicOr(&c.ctrl->status, 0x10u);
+}
+
+// kFlagFar and kFlagFast of a stray that moved by `move` cells (window bases 1..4 are the tile's, 0 and 5 one cell out;
+// the windows end three cells from their middle). The pass that follows still reads this list, so a particle as close to
+// the window's end as it moves, or a quarter cell, asks for a sort.
+__device__ __forceinline__ unsigned stray_flags(int l0, int l1, int l2, const float t[3], float move) {
+  const float e = fmaxf(fmaxf(fabsf(static_cast<float>(l0) + t[0] - 3.5f), fabsf(static_cast<float>(l1) + t[1] - 3.5f)),
+                        fabsf(static_cast<float>(l2) + t[2] - 3.5f));
+  return e + fmaxf(0.25f, move) > 3.f ? kFlagFar | (move > 0.5f ? kFlagFast : 0u) : 0u;
 }
 
 // Phase A of one particle (home slot `home`, payload row j): G2P from the staged window, F update,
 // fixed-point advection and the constitutive update / return map (src/three/mpm.js:107-131), or,
 // for the P2G pass and pinned particles, the stress of the stored state; then the scatter payload
 // bucketed by its new stencil base in the shared window (pay, meta, hist), and the CFL terms.
-// Writes the particle's new state and returns its next sort key (all ones unless want is set); stray: its new base
-// lies outside the tile.
+// Writes the particle's new state and returns its next sort key (all ones unless want is set). drift: 1 if its new base
+// lies outside the tile; from the P2G pass its speed in cells per second (float bits).
 // NEWTON (the Newton-gated return mode): a Johnson-Cook trial stress above the initial flow stress
 // takes the gated refinement from u0 = 1 - flow(ep, 0, T) / q instead of the bisection, which stays
 // the fallback; gate[0] / gate[1] count the returns accepted / sent to the bisection.
@@ -1110,7 +1125,7 @@ __device__ __forceinline__ unsigned particle_phase_a(const Ctx& c, const SceneDe
                                                      unsigned home, unsigned j, float dt, int nxt, float4* pay,
                                                      unsigned* meta, int* hist, float& wave_acc, float& grad_acc,
                                                      unsigned& flags_acc, double& work_acc, bool store_vc,
-                                                     bool want, bool& stray, unsigned* gate = nullptr) {
+                                                     bool want, unsigned& drift, unsigned* gate = nullptr) {
   static_assert(!NEWTON || (!HEAT && !AUX && PASS != kPassP2G), "Newton-gated returns: J2-type laws, gather passes");
   constexpr bool SCATTER = PASS != kPassG2P;
   constexpr bool GATHER = PASS != kPassP2G;
@@ -1234,9 +1249,11 @@ __device__ __forceinline__ unsigned particle_phase_a(const Ctx& c, const SceneDe
     }
     ep += co.dep;
     T += co.dT;
+    // the history laws' registers run out (36 bytes of spills) with the report between the stores, the others' before them
+    if (SCATTER && AUX) report_long_move(c, tc, home, q, v, dt);
 #pragma unroll
     for (int e = 0; e < 9; ++e) c.p.Dc[e][home] = D[e];
-    if (SCATTER) report_long_move(c, tc, home, q, v, dt);
+    if (SCATTER && !AUX) report_long_move(c, tc, home, q, v, dt);
     c.p.qx[home] = q[0]; c.p.qy[home] = q[1]; c.p.qz[home] = q[2];
     // v and C: the fused pass scatters the ones it just gathered and never reads the stored copies,
     // so it stores them only on the call's last substep (downloads, ledgers, frames, regularisation
@@ -1259,6 +1276,7 @@ __device__ __forceinline__ unsigned particle_phase_a(const Ctx& c, const SceneDe
 #pragma unroll
     for (int e = 0; e < 9; ++e) Dc[e] = D[e];
     co = constitutive_update_t<AUX>(mt, Dc, ep, aux, T, V / m, false, 0.f, xp);
+    if (PASS == kPassP2G && !pinned) drift = fbits(largest_move(v, 1.f, tc.invH));
   }
   if (SCATTER) {
     // payload of the scatter: fraction t, m, m v, m C h, -4 V / h tau
@@ -1281,8 +1299,9 @@ __device__ __forceinline__ unsigned particle_phase_a(const Ctx& c, const SceneDe
               l2 = nb[2] - (tc.tile[2] * kTile - 1);
     const bool in_w = l0 >= 0 && l0 <= kWinS - 3 && l1 >= 0 && l1 <= kWinS - 3 && l2 >= 0 && l2 <= kWinS - 3;
     if (PASS == kPassG2P2G && in_w) {
-      stray = (((l0 - 1) | (l1 - 1) | (l2 - 1)) & ~3) != 0;
-      if (stray && near_window_end(l0, t[0], l1, t[1], l2, t[2])) flags |= kFlagFar;
+      const bool stray = (((l0 - 1) | (l1 - 1) | (l2 - 1)) & ~3) != 0;
+      drift = stray ? 1u : 0u;
+      if (stray) flags |= stray_flags(l0, l1, l2, t, largest_move(v, dt, tc.invH));
     }
     if (in_w && !pinned) {
       const int bucket = (l2 * 6 + l1) * 6 + l0;
@@ -1302,8 +1321,8 @@ __device__ __forceinline__ unsigned particle_phase_a(const Ctx& c, const SceneDe
     } else {
       meta[j] = kMetaInvalid;
       if (!in_w) {
-        stray = true;
-        flags |= kFlagFar;
+        drift = 1u;
+        flags |= kFlagFar | (largest_move(v, dt, tc.invH) > 0.5f ? kFlagFast : 0u);
         if (c.ctrl->list_age == 0u) flags |= 0x10u;  // the window is that of the particle's own tile
       }
       // copies scoped to this rare branch: the arrays passed to the out-of-line scatter would
@@ -1372,7 +1391,7 @@ __device__ __forceinline__ unsigned particle_phase_a_learned(const Ctx& c, const
                                                              const float4* vwin, bool live, unsigned home, unsigned j,
                                                              float dt, int nxt, float4* pay, unsigned* meta, int* hist,
                                                              float& wave_acc, float& grad_acc, unsigned& flags_acc,
-                                                             double& work_acc, bool store_vc, bool want, bool& stray,
+                                                             double& work_acc, bool store_vc, bool want, unsigned& drift,
                                                              unsigned* gate) {
   constexpr bool SCATTER = PASS != kPassG2P;
   static_assert(PASS != kPassP2G, "the learned mode changes only returns");
@@ -1515,8 +1534,9 @@ __device__ __forceinline__ unsigned particle_phase_a_learned(const Ctx& c, const
               l2 = nb[2] - (tc.tile[2] * kTile - 1);
     const bool in_w = l0 >= 0 && l0 <= kWinS - 3 && l1 >= 0 && l1 <= kWinS - 3 && l2 >= 0 && l2 <= kWinS - 3;
     if (PASS == kPassG2P2G && in_w) {
-      stray = (((l0 - 1) | (l1 - 1) | (l2 - 1)) & ~3) != 0;
-      if (stray && near_window_end(l0, t[0], l1, t[1], l2, t[2])) flags |= kFlagFar;
+      const bool stray = (((l0 - 1) | (l1 - 1) | (l2 - 1)) & ~3) != 0;
+      drift = stray ? 1u : 0u;
+      if (stray) flags |= stray_flags(l0, l1, l2, t, largest_move(v, dt, tc.invH));
     }
     if (in_w && !pinned) {
       const int bucket = (l2 * 6 + l1) * 6 + l0;
@@ -1534,8 +1554,8 @@ __device__ __forceinline__ unsigned particle_phase_a_learned(const Ctx& c, const
     } else {
       meta[j] = kMetaInvalid;
       if (!in_w) {
-        stray = true;
-        flags |= kFlagFar;
+        drift = 1u;
+        flags |= kFlagFar | (largest_move(v, dt, tc.invH) > 0.5f ? kFlagFast : 0u);
         if (c.ctrl->list_age == 0u) flags |= 0x10u;  // the window is that of the particle's own tile
       }
       // copies scoped to this rare branch: the arrays passed to the out-of-line scatter would
@@ -1747,32 +1767,33 @@ __global__ void __launch_bounds__(kBlock, 2) k_particles(const __grid_constant__
         unsigned key = kNone;
         float wave = 0.f, grad = 0.f;
         unsigned flags = 0;
-        bool stray = false;
+        unsigned drift = 0u;
         const SceneDev& sc = c.scenes[sm.item[cb].w];
         if constexpr (JC == 1) {
           // every lane of a warp with a live particle takes part in its network evaluation
           const unsigned home = !live ? c.p.perm[sm.item[cb].y + r0]
                                       : (r0 == 0 && jj < kPf * kBlock) ? sm.pfs[j] : c.p.perm[sm.item[cb].y + r0 + j];
           key = particle_phase_a_learned<PASS>(c, sc, tc, sm.mt, single, sm.vwin, live, home, j, tc.dt, nxt, sm.pay,
-                                               sm.meta, sm.hist, wave, grad, flags, sm.work_sum, store_vc, want, stray,
+                                               sm.meta, sm.hist, wave, grad, flags, sm.work_sum, store_vc, want, drift,
                                                sm.gate);
         } else if (live) {
           const unsigned home = (r0 == 0 && jj < kPf * kBlock) ? sm.pfs[j] : c.p.perm[sm.item[cb].y + r0 + j];
           key = particle_phase_a<PASS, HEAT, AUX, JC == 2>(c, sc, tc, sm.mt, single, sm.vwin, home, j, tc.dt, nxt, sm.pay,
                                                            sm.meta, sm.hist, wave, grad, flags, sm.work_sum, store_vc,
-                                                           want, stray, sm.gate);
+                                                           want, drift, sm.gate);
         }
         if (want) count_key(c, key);
         // CFL maxima, status flags and strays of the tile
         const unsigned wb = __reduce_max_sync(0xffffffffu, fbits(wave));
         const unsigned gb = __reduce_max_sync(0xffffffffu, fbits(grad));
         const unsigned fl = __reduce_or_sync(0xffffffffu, flags);
-        const unsigned out = __ballot_sync(0xffffffffu, stray);
+        const unsigned out = PASS == kPassP2G ? __reduce_max_sync(0xffffffffu, drift) : __popc(__ballot_sync(0xffffffffu, drift != 0u));
         if ((threadIdx.x & 31) == 0) {
           atomicMax(&sm.red[0], wb);
           atomicMax(&sm.red[1], gb);
           if (fl) atomicOr(&sm.red[2], fl);
-          if (out) atomicAdd(&sm.red[3], __popc(out));
+          if (PASS == kPassP2G) atomicMax(&sm.red[3], out);
+          if (PASS != kPassP2G && out) atomicAdd(&sm.red[3], out);
         }
       }
       // the last thread claims the next tile (a full tile has about 3 x 64 phase-B tasks, so its warp
@@ -1805,9 +1826,11 @@ __global__ void __launch_bounds__(kBlock, 2) k_particles(const __grid_constant__
       const unsigned scene = sm.item[cb].w;
       atomicMax(&c.wave_max[scene], sm.red[0]);
       atomicMax(&c.grad_max[scene], sm.red[1]);
-      if (sm.red[2] & ~kFlagFar) atomicOr(&ct->status, sm.red[2] & ~kFlagFar);
-      if (sm.red[2] & kFlagFar) atomicOr(&ct->far_strays, 1u);
-      if (sm.red[3]) atomicAdd(&ct->strays, sm.red[3]);
+      const unsigned drift = sm.red[2] & (kFlagFar | kFlagFast);
+      if (sm.red[2] & ~(kFlagFar | kFlagFast)) atomicOr(&ct->status, sm.red[2] & ~(kFlagFar | kFlagFast));
+      if (drift) atomicOr(&ct->far_strays, drift);
+      if (PASS == kPassP2G) atomicMax(&ct->first_speed, sm.red[3]);
+      if (PASS != kPassP2G && sm.red[3]) atomicAdd(&ct->strays, sm.red[3]);
       sm.red[0] = sm.red[1] = sm.red[2] = sm.red[3] = 0u;
     }
     if (SCATTER) flush_window(c, c.scenes[sm.item[cb].w], sm, nxt, tc.tile);
@@ -2033,12 +2056,12 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_particles_ws(const __grid_con
         for (unsigned jj = 0; jj < nround; jj += kWsGroup) {
           const unsigned j = jj + tid;
           unsigned key = 0xffffffffu;
-          bool stray = false;
+          unsigned drift = 0u;
           if (j < nround) {
             const unsigned home = c.p.perm[it.y + r0 + j];
             key = particle_phase_a<PASS, HEAT, AUX>(c, sc, tc, sm.mt, single, sm.vwin[cb], home, j, dt, nxt, sm.pay[s],
                                          sm.meta[s], sm.hist[s], wave_acc, grad_acc, flags_acc, sm.work_sum, store_vc, true,
-                                         stray);
+                                         drift);
           }
           if (PASS == kPassG2P2G) count_key(c, key);
         }
@@ -2060,7 +2083,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_particles_ws(const __grid_con
         s ^= 1;
       }
       if (stop) break;
-      group_reduce_item(c, scene, wave_acc, grad_acc, flags_acc & ~kFlagFar, sm.red, tid);
+      group_reduce_item(c, scene, wave_acc, grad_acc, flags_acc & ~(kFlagFar | kFlagFast), sm.red, tid);
       cb ^= 1;
     }
     // sentinel stage: the consumer leaves after it. A group that stopped early first lets its own

@@ -180,3 +180,53 @@ def test_overflow_status_follows_a_particles_own_tile(x0, cells, gravity, dts):
         assert sol.status() == expected, (before, after)
         before = after
     sol.close()
+
+
+# around and past half a cell per substep, where two substeps outrun the windows of one list, and past a whole cell
+@pytest.mark.parametrize("cells_per_step", [.49, .51, .95, 1.6])
+def test_lists_follow_a_fast_body(cells_per_step):
+    d = Domain(lower=(0, 0, 0), upper=(1, 1, 1), H=1 / 32)
+    mat = Material.from_young(0, 1e5, .3, density=1000.0)
+    x = scenes.block_particles(d, (2, 2, 2), (9, 7, 8), 5)
+    dt, steps = 1e-5, 12
+    v = cells_per_step * d.H / dt
+    sc = scenes._scene("fast", d, [mat], x, (v, .7 * v, .4 * v))
+    sol = Solver(sc.domain, sc.n)
+    sol.upload(sc)
+    st = orc.state_from_scene(sc)
+    for k in (1, 4, 7):  # the first substep after a fresh scatter, and kept lists between calls
+        sol.step_fixed(dt, k)
+        for _ in range(k):
+            st.step(dt)
+    out = sol.download(("x", "F"))
+    # as for the slower body: a position is rounded to H / 2^22 each substep, each substep adds dt v with FP32's v
+    assert np.max(np.abs(out["x"] - st.x)) <= 1e-6 + steps * d.H / 2 ** 23 + 4 * steps * dt * v * 2.0 ** -24
+    assert np.max(np.abs(out["F"] - st.F)) <= 2e-6 * 40 * cells_per_step
+    assert sol.status() == (0x10 if cells_per_step > 1 else 0)
+    sol.close()
+
+
+def test_a_fast_body_keeps_to_the_windows():
+    """Particles out of the windows are scattered one by one in global memory, at several times the cost of the
+    pass: a body at .9 cells per substep takes about the time of one at .3, not more than twice it."""
+    d = Domain(lower=(0, 0, 0), upper=(1, 1, 1), H=1 / 128)
+    x = scenes.block_particles(d, (3, 3, 3), (67, 19, 35), 5)
+    sc = scenes._scene("fast", d, [Material.from_young(0, 1e5, .3, density=1000.0)], x, (0, 0, 0))
+    dt, took = 1e-6, {}
+    for cells in (.3, .9):
+        sc.v[:] = np.array([1, .7, .4]) * cells * d.H / dt
+        sol = Solver(d, sc.n)
+        sol.upload(sc)
+        sol.snapshot()
+        sol.profile()
+        times = []
+        for _ in range(4):
+            sol.rollback()
+            sol.step_fixed(dt, 1)
+            sol.profile_read()
+            sol.step_fixed(dt, 20)
+            ms, count = sol.profile_read()["g2p2g"]
+            times.append(ms / count)
+        took[cells] = min(times)
+        sol.close()
+    assert took[.9] <= 2 * took[.3], took
