@@ -489,7 +489,7 @@ static int prepare_grid(mpm_handle* h) {
   { ProfScope ps(h, -1); mpm::launch_control_init(c, h->stream); }
   MPM_CUDA(h, cudaMemsetAsync(c.s.count, 0, sizeof(unsigned) * (c.total_tiles + 1), h->stream));
   { ProfScope ps(h, 6); mpm::launch_keys(c, h->stream); }
-  { ProfScope ps(h, 3); mpm::launch_scan(c, h->stream, true); }
+  { ProfScope ps(h, 3); mpm::launch_scan(c, h->stream); }
   { ProfScope ps(h, 4); mpm::launch_sort_scatter(c, h->stream); }
   if (h->reorder_pending) {
     ProfScope ps(h, -1);

@@ -39,11 +39,6 @@ constexpr int kBlock = 256;                      // threads per CTA in the parti
 constexpr int kMaxScenes = 4096;
 constexpr int kMaxMaterials = 4096;
 
-// Largest tile count whose scan k_open does by itself, in the few substeps that sort; above it k_scan is
-// launched in every substep. Substep at 110,592 particles and 32,768 tiles, k_scan against k_open: at rest 43.1 and
-// 40.3 us, at .02 cells a substep 50.4 and 50.5, at .3 cells (sorted every time) 53.5 and 57.2.
-constexpr int kOpenScanTiles = 32768;
-
 enum StepMode : int { kModeFixed = 0, kModeRequested = 1, kModeCfl = 2 };
 
 struct SceneDev {
@@ -207,7 +202,7 @@ MaterialDev material_to_device(const mpm_material& m);
 // Launch wrappers (mpm_kernels.cu)
 void launch_control_init(const Ctx& c, cudaStream_t st);
 void launch_keys(const Ctx& c, cudaStream_t st);
-void launch_scan(const Ctx& c, cudaStream_t st, bool initial);
+void launch_scan(const Ctx& c, cudaStream_t st);
 void launch_wait_probe(cudaStream_t st, unsigned* out, long long limit);
 void launch_sort_scatter(const Ctx& c, cudaStream_t st);
 void launch_p2g(const Ctx& c, cudaStream_t st, int grid_blocks);

@@ -370,12 +370,6 @@ constexpr int kScanThreads = 1024;
 constexpr int kScanPer = 4;
 constexpr int kScanChunk = kScanThreads * kScanPer;  // 4096 tiles per block
 
-// Exclusive scans of count[0..T] into start (block-local) + block_off (per 4096 tiles), and of the
-// tiles' item counts into rank + block_rank (a tile's place in the work list, which so comes out in
-// tile-key order; an empty tile has none). The last block to finish scans the block sums (threadfence + ticket) and sets
-// the work list's length.
-// The new list becomes the one that passes read. initial: a first sort; otherwise after a scatter pass,
-// if it wrote keys.
 __device__ __forceinline__ uint2 warp_incl_scan2(uint2 v, int lane) {
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -392,13 +386,15 @@ __device__ __forceinline__ uint2 warp_incl_scan2(uint2 v, int lane) {
 // Work items of a tile with cnt particles (0 for an empty tile).
 __device__ __forceinline__ unsigned tile_items(unsigned cnt, int shift) { return (cnt + (1u << shift) - 1u) >> shift; }
 
-__global__ void __launch_bounds__(kScanThreads) k_scan(Ctx c, int initial) {
-  if (initial ? c.ctrl->done != 0 : c.ctrl->sort_active == 0) return;
-  if (c.ctrl->status & 0x8u) return;
+// Exclusive scans of count[0..T] into start (block-local) + block_off (per 4096 tiles), and of the
+// tiles' item counts into rank + block_rank (a tile's place in the work list, which so comes out in
+// tile-key order; an empty tile has none), by `blocks` CTAs of which this is `block`. The last block to finish scans
+// the block sums (threadfence + ticket) and sets the work list's length. The new list becomes the one that passes read.
+__device__ __forceinline__ void scan_tiles(const Ctx& c, int block, int blocks) {
   __shared__ uint2 warp_sums[32];
   __shared__ bool last;
   const int T = c.total_tiles + 1;
-  const int base = blockIdx.x * kScanChunk + threadIdx.x * kScanPer;
+  const int base = block * kScanChunk + threadIdx.x * kScanPer;
   unsigned v[kScanPer];
   uint2 sum = make_uint2(0u, 0u);
 #pragma unroll
@@ -428,23 +424,31 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(Ctx c, int initial) {
     run.x += v[k];
     run.y += tile_items(v[k], c.split_shift);
   }
+  auto publish = [&](unsigned items) {
+    const unsigned list = c.ctrl->sort_list ^ 1u;
+    c.ctrl->work_count[list] = items;
+    c.ctrl->sort_list = list;
+    c.ctrl->in_place = 0u;
+  };
   if (threadIdx.x == kScanThreads - 1) {  // block totals
-    c.s.block_off[blockIdx.x] = run.x;
-    c.s.block_rank[blockIdx.x] = run.y;
+    c.s.block_off[block] = blocks > 1 ? run.x : 0u;
+    c.s.block_rank[block] = blocks > 1 ? run.y : 0u;
+    if (blocks == 1) publish(run.y);
   }
+  if (blocks == 1) return;
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) last = (atomicAdd(&c.ctrl->scan_ticket, 1u) == gridDim.x - 1);
+  if (threadIdx.x == 0) last = (atomicAdd(&c.ctrl->scan_ticket, 1u) == static_cast<unsigned>(blocks) - 1);
   __syncthreads();
   if (!last) return;
   __threadfence();
-  // last block: exclusive scan of the block totals (gridDim.x <= 1024 * 64 blocks)
+  // last block: exclusive scan of the block totals
   __shared__ uint2 carry;
   if (threadIdx.x == 0) carry = make_uint2(0u, 0u);
   __syncthreads();
-  for (int b0 = 0; b0 < (int)gridDim.x; b0 += kScanThreads) {
+  for (int b0 = 0; b0 < blocks; b0 += kScanThreads) {
     const int b = b0 + threadIdx.x;
-    const uint2 x = (b < (int)gridDim.x)
+    const uint2 x = (b < blocks)
                         ? make_uint2(*((volatile unsigned*)&c.s.block_off[b]), *((volatile unsigned*)&c.s.block_rank[b]))
                         : make_uint2(0u, 0u);
     const uint2 inc = warp_incl_scan2(x, lane);
@@ -457,7 +461,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(Ctx c, int initial) {
     }
     __syncthreads();
     const uint2 excl = make_uint2(carry.x + warp_sums[wid].x + inc.x - x.x, carry.y + warp_sums[wid].y + inc.y - x.y);
-    if (b < (int)gridDim.x) {
+    if (b < blocks) {
       c.s.block_off[b] = excl.x;
       c.s.block_rank[b] = excl.y;
     }
@@ -466,117 +470,39 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(Ctx c, int initial) {
     __syncthreads();
   }
   if (threadIdx.x == 0) {
-    const unsigned list = c.ctrl->sort_list ^ 1u;
-    c.ctrl->work_count[list] = carry.y;
-    c.ctrl->sort_list = list;
-    c.ctrl->in_place = 0u;
+    publish(carry.y);
     c.ctrl->scan_ticket = 0;
   }
 }
 
-void launch_scan(const Ctx& c, cudaStream_t st, bool initial) {
-  const int blocks = (c.total_tiles + 1 + kScanChunk - 1) / kScanChunk;
-  k_scan<<<blocks, kScanThreads, 0, st>>>(c, initial ? 1 : 0);
+__host__ __device__ __forceinline__ int scan_blocks(const Ctx& c) { return (c.total_tiles + 1 + kScanChunk - 1) / kScanChunk; }
+
+// The scan of a first sort.
+__global__ void __launch_bounds__(kScanThreads) k_scan(Ctx c) {
+  if (c.ctrl->done == 0 && !(c.ctrl->status & 0x8u)) scan_tiles(c, blockIdx.x, gridDim.x);
 }
+
+void launch_scan(const Ctx& c, cudaStream_t st) { k_scan<<<scan_blocks(c), kScanThreads, 0, st>>>(c); }
 
 __device__ __forceinline__ unsigned tile_start(const Ctx& c, unsigned k) {
   return c.s.start[k] + c.s.block_off[k / kScanChunk];
 }
 
-// The same scan by one CTA, PER tiles a thread and round, after a scatter pass that wrote keys (grids of at most
-// kOpenScanTiles tiles): with most passes keeping their lists it runs once in tens of substeps, where a launch of its own
-// would cost every substep. start and rank come out global here, the block offsets zero.
-template <int PER>
-__device__ __forceinline__ void scan_tiles(const Ctx& c) {
-  __shared__ uint2 sums[kScanThreads / 32];
-  const int T = c.total_tiles, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  uint2 carry = make_uint2(0u, 0u);
-  for (int r0 = 0; r0 < T; r0 += kScanThreads * PER) {
-    const int base = r0 + threadIdx.x * PER;
-    unsigned v[PER];
-    uint2 sum = make_uint2(0u, 0u);
-#pragma unroll
-    for (int q = 0; q < PER; q += 4) {
-      if (base + q + 4 <= T) {
-        const uint4 x = *reinterpret_cast<const uint4*>(c.s.count + base + q);
-        v[q] = x.x; v[q + 1] = x.y; v[q + 2] = x.z; v[q + 3] = x.w;
-      } else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) v[q + e] = base + q + e < T ? c.s.count[base + q + e] : 0u;
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < PER; ++q) {
-      sum.x += v[q];
-      sum.y += tile_items(v[q], c.split_shift);
-    }
-    const uint2 incl = warp_incl_scan2(sum, lane);
-    __syncthreads();  // sums of the round before are read
-    if (lane == 31) sums[wid] = incl;
-    __syncthreads();
-    uint2 run = make_uint2(carry.x + incl.x - sum.x, carry.y + incl.y - sum.y);
-    for (int w = 0; w < kScanThreads / 32; ++w) {
-      const uint2 x = sums[w];
-      if (w < wid) {
-        run.x += x.x;
-        run.y += x.y;
-      }
-      carry.x += x.x;
-      carry.y += x.y;
-    }
-#pragma unroll
-    for (int q = 0; q < PER; q += 4) {
-      unsigned st[4], rk[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        st[e] = run.x;
-        rk[e] = run.y;
-        run.x += v[q + e];
-        run.y += tile_items(v[q + e], c.split_shift);
-      }
-      if (base + q + 4 <= T) {
-        *reinterpret_cast<uint4*>(c.s.start + base + q) = make_uint4(st[0], st[1], st[2], st[3]);
-        *reinterpret_cast<uint4*>(c.s.rank + base + q) = make_uint4(rk[0], rk[1], rk[2], rk[3]);
-      } else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if (base + q + e < T) {
-            c.s.start[base + q + e] = st[e];
-            c.s.rank[base + q + e] = rk[e];
-          }
-      }
-    }
-  }
-  for (int b = threadIdx.x; b * kScanChunk <= T; b += kScanThreads) c.s.block_off[b] = c.s.block_rank[b] = 0u;
-  if (threadIdx.x == 0) {
-    c.s.start[T] = carry.x;
-    c.s.rank[T] = carry.y;
-    const unsigned list = c.ctrl->sort_list ^ 1u;
-    c.ctrl->work_count[list] = carry.y;
-    c.ctrl->sort_list = list;
-    c.ctrl->in_place = 0u;
-  }
-}
-
-// Between two particle passes. scan: a scatter pass came before, and if it wrote keys its counts are
-// scanned; begin: opens the next substep.
-__global__ void __launch_bounds__(kScanThreads) k_open(Ctx c, int begin, int scan) {
-  if (scan && c.ctrl->sort_active != 0 && !(c.ctrl->status & 0x8u)) {
-    if (c.total_tiles <= kScanChunk)
-      scan_tiles<kScanPer>(c);
-    else
-      scan_tiles<16>(c);
-  }
-  __syncthreads();
-  if (begin) begin_substep(c);
+// Between two particle passes: the first CTA opens the next substep (begin), the others scan the tile counts if the
+// scatter pass before wrote keys, a CTA per 4,096 tiles. With most passes keeping their lists the scan runs once in tens
+// of substeps, where a launch of its own would cost every one: 262,144 particles on 39,304 tiles at rest 55.8 us a
+// substep with that launch, 52.6 so. One CTA for all tiles, before the opening, cost what moves: 110,592 particles
+// on 32,768 tiles 34.3 us at rest, 54.3 at .3 cells a substep and 60.9 at .9; so 32.6, 48.2 and 50.9.
+__global__ void __launch_bounds__(kScanThreads) k_open(Ctx c, int begin) {
+  if (begin && blockIdx.x == 0)
+    begin_substep(c);
+  else if (c.ctrl->sort_active != 0 && !(c.ctrl->status & 0x8u))
+    scan_tiles(c, static_cast<int>(blockIdx.x) - begin, static_cast<int>(gridDim.x) - begin);
 }
 
 void launch_open(const Ctx& c, cudaStream_t st, bool begin, bool scan) {
-  if (scan && c.total_tiles > kOpenScanTiles) {
-    launch_scan(c, st, false);
-    scan = false;
-  }
-  if (begin || scan) k_open<<<1, kScanThreads, 0, st>>>(c, begin ? 1 : 0, scan ? 1 : 0);
+  const int blocks = (begin ? 1 : 0) + (scan ? scan_blocks(c) : 0);
+  if (blocks > 0) k_open<<<blocks, kScanThreads, 0, st>>>(c, begin ? 1 : 0);
 }
 
 // perm[start(k) + rank] = home slot; the group that claims a tile first writes its work item.

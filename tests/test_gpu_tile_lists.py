@@ -230,3 +230,27 @@ def test_a_fast_body_keeps_to_the_windows():
         took[cells] = min(times)
         sol.close()
     assert took[.9] <= 2 * took[.3], took
+
+
+# the scan of the tile counts over one, two and ten CTAs, with bodies that a run sorts again and again
+@pytest.mark.parametrize("grid", [32, 64, 128])
+@pytest.mark.parametrize("cells_per_step", [.05, .7])
+def test_lists_follow_a_body_on_grids_of_many_tiles(grid, cells_per_step):
+    d = Domain(lower=(0, 0, 0), upper=(1, 1, 1), H=1 / grid)
+    corner = grid - 26
+    x = np.concatenate([scenes.block_particles(d, (2, 2, 2), (9, 7, 8), 5), scenes.block_particles(d, (corner,) * 3, (corner + 5,) * 3, 6)])
+    dt, steps = 1e-5, 16
+    v = cells_per_step * d.H / dt
+    sc = scenes._scene("two bodies", d, [Material.from_young(0, 1e5, .3, density=1000.0)], x, (v, .7 * v, .4 * v))
+    sol = Solver(sc.domain, sc.n)
+    sol.upload(sc)
+    st = orc.state_from_scene(sc)
+    sol.step_fixed(dt, steps)
+    for _ in range(steps):
+        st.step(dt)
+    out = sol.download(("x", "F"))
+    # as above: positions rounded to H / 2^22, dt v with FP32's v each substep
+    assert np.max(np.abs(out["x"] - st.x)) <= 1e-6 + steps * d.H / 2 ** 23 + 4 * steps * dt * v * 2.0 ** -24
+    assert np.max(np.abs(out["F"] - st.F)) <= 2e-6 * 40 * cells_per_step
+    assert sol.status() == 0
+    sol.close()
