@@ -592,6 +592,12 @@ int smpm_stats_get(smpm_handle* h, const smpm_sim* s, smpm_stats* out);  /* Soli
  * stableStep), each applying the body force of Simulation.substep (src/simulation.js:270-288)
  * before the step. dt is clamped to [0, 0.05]. One host round trip per call. */
 int smpm_frame(smpm_handle* h, const smpm_sim* s, double dt, int32_t* substeps, double* advanced);
+/* Self-check of the bounded waits of smpm_frame's one-launch form: its grid barriers give up after about a second, and
+ * the frame is then taken again from its start in separate launches, as it is when the launch is refused. Reports
+ * how many frames gave up so far (frames_given_up may be NULL) and lets the barriers of later frames from the
+ * from_barrier-th on (0: the first; one before the first substep and three in each) give up after `polls` polls, 0: about a
+ * second again. */
+int smpm_check_bounded_wait(smpm_handle* h, int32_t from_barrier, int64_t polls, int64_t* frames_given_up);
 /* Read / write the eight deformation fields (f00 f01 f10 f11 c00 c01 c10 c11) of slots
  * [0, n) as fields[8][n] doubles. */
 int smpm_get_fields(smpm_handle* h, int64_t n, double* fields);

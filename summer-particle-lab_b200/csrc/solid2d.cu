@@ -44,11 +44,19 @@ struct Ctrl2 {
   unsigned wave_bits, grad_bits;  // stableStep maxima (non-negative floats compare as uints)
   // stats reduction
   unsigned count, minj_key, maxj_key, strain_bits;
-  // k2_frame: arrivals at the grid barrier, a barrier wait that gave up, and by substep parity the
+  // k2_frame: arrivals at the grid barrier, how the frame ended (kFrame*), and by substep parity the
   // stableStep maxima and the active-node count
-  unsigned barrier, timeout;
+  unsigned barrier, verdict;
   unsigned wave2[2], grad2[2];
   int active2[2];
+};
+
+// How a k2_frame ended: not yet, past its last barrier, or given up at a barrier.
+constexpr unsigned kFrameOpen = 0u, kFrameDone = 1u, kFrameGaveUp = 2u;
+
+// Polls after which a grid barrier of k2_frame gives up, about a second; from barrier `from` on (0: the first) `polls`.
+struct Wait2 {
+  unsigned from = 0xffffffffu, polls = 1u << 21;
 };
 
 struct Params2 {
@@ -324,24 +332,34 @@ __global__ void __launch_bounds__(kThreads) k2_g2p(Dev2 d, Params2 p, int frame)
   }
 }
 
-// Grid barrier of a cooperative launch: round counts the barriers passed. Bounded: after about a second
-// of polling it reports false, and the kernel leaves.
-__device__ bool grid_barrier(Ctrl2* c, unsigned& round) {
+// Grid barrier of a cooperative launch: round counts the barriers passed. Bounded: a wait that gives up ends the
+// frame, unless a CTA is past its last barrier already, which takes all to have arrived there.
+__device__ bool grid_barrier(Ctrl2* c, unsigned& round, const Wait2& w) {
   __shared__ int ok;
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
     atomicAdd(&c->barrier, 1u);
+    const unsigned limit = round >= w.from ? w.polls : Wait2{}.polls;
     const unsigned target = ++round * gridDim.x;
     ok = 0;
-    for (int i = 0; i < (1 << 21); ++i)
+    for (unsigned i = 0; i < limit; ++i)
       if (*(volatile unsigned*)&c->barrier >= target) {
         ok = 1;
         break;
       }
-    if (!ok) atomicOr(&c->timeout, 1u);
+    if (!ok) ok = atomicCAS(&c->verdict, kFrameOpen, kFrameGaveUp) == kFrameDone;
     __threadfence();
   }
+  __syncthreads();
+  return ok != 0;
+}
+
+// Whether the frame's results are to be stored: a CTA past the last barrier closes the frame for all, unless one
+// that gave up there has. So either all CTAs store or none does.
+__device__ bool close_frame(Ctrl2* c) {
+  __shared__ int ok;
+  if (threadIdx.x == 0) ok = atomicCAS(&c->verdict, kFrameOpen, kFrameDone) != kFrameGaveUp;
   __syncthreads();
   return ok != 0;
 }
@@ -350,7 +368,7 @@ __device__ bool grid_barrier(Ctrl2* c, unsigned& round) {
 // substeps as k2_stable and the k2_p2g, k2_grid, k2_g2p sequence, separated by grid barriers. The reference's
 // 16,000 particles are bound by launches and host checks: four substeps took 47 us in 13 kernels with their gaps,
 // and each frame copied its control block back at least once more. Node sums and velocities are read from L2.
-__global__ void __launch_bounds__(kThreads) k2_frame(Dev2 d, Params2 p) {
+__global__ void __launch_bounds__(kThreads) k2_frame(Dev2 d, Params2 p, Wait2 wait) {
   Ctrl2* ct = d.ctrl;
   const int i = blockIdx.x * kThreads + threadIdx.x;
   const bool live = i < p.count && solid(p, d.material[i]);
@@ -369,7 +387,7 @@ __global__ void __launch_bounds__(kThreads) k2_frame(Dev2 d, Params2 p) {
   block_max2(wave, grad, &ct->wave2[0], &ct->grad2[0]);
   double remaining = ct->remaining, h_last = 0.0;
   int steps = 0;
-  if (!grid_barrier(ct, round)) return;
+  if (!grid_barrier(ct, round, wait)) return;
   while (true) {
     const int par = steps & 1;
     // src/solid-mpm.js:45, src/simulation.js:250-253
@@ -404,20 +422,21 @@ __global__ void __launch_bounds__(kThreads) k2_frame(Dev2 d, Params2 p) {
       stencil2(x, y, s);
       scatter2(d, s, p, h, F, C, m, V0, vx, vy, pin);
     }
-    if (!grid_barrier(ct, round)) return;
+    if (!grid_barrier(ct, round, wait)) return;
     int active = 0;
     for (int n = i; n < kNodes; n += gridDim.x * kThreads) active += update_node2(d, p, n);
     for (int o = 16; o; o >>= 1) active += __shfl_xor_sync(0xffffffffu, active, o);
     if ((threadIdx.x & 31) == 0 && active) atomicAdd(&ct->active2[par], active);
-    if (!grid_barrier(ct, round)) return;
+    if (!grid_barrier(ct, round, wait)) return;
     if (live && !pin) gather2(d, s, p, h, x, y, vx, vy, F, C);
     wave = grad = 0;
     if (live) stable_terms(p, F, C, vx, vy, wave, grad);
     block_max2(wave, grad, &ct->wave2[par ^ 1], &ct->grad2[par ^ 1]);
     remaining -= hd;
     ++steps;
-    if (!grid_barrier(ct, round)) return;
+    if (!grid_barrier(ct, round, wait)) return;
   }
+  if (!close_frame(ct)) return;
   if (live) {
     d.x[i] = x; d.y[i] = y; d.vx[i] = vx; d.vy[i] = vy;
     d.F[i] = F;
@@ -477,6 +496,8 @@ struct smpm_handle {
   size_t stage_bytes = 0;      // size of that block
   unsigned mask[8] = {};
   int frame_blocks = 0;  // CTAs of k2_frame that are resident at once (0: no cooperative launch)
+  Wait2 wait;            // of the frame's grid barriers
+  int frames_given_up = 0;
   int substeps = 0;  // SolidMPM.substeps: set by a frame
   int nodes = 0;     // SolidMPM.activeNodes: set by every grid pass
   std::string err;
@@ -575,22 +596,38 @@ int upload_sim(smpm_handle* h, const smpm_sim* s, double remaining, double step)
   return h->cuda(e, "copy particles in");
 }
 
-int download_sim(smpm_handle* h, const smpm_sim* s) {
+// The control block and, in a staged call, the particle arrays behind it to the pinned block.
+int fetch_sim(smpm_handle* h, const smpm_sim* s) {
+  size_t total = 0;
+  const size_t back = lay_out(h, (size_t)s->count, &total);
+  cudaError_t e = cudaMemcpyAsync(h->host_ctrl, h->d.ctrl, total <= h->stage_bytes ? back : sizeof(Ctrl2), cudaMemcpyDeviceToHost, h->stream);
+  e = e ? e : cudaStreamSynchronize(h->stream);
+  return h->cuda(e, "copy particles out");
+}
+
+// What fetch_sim brought to the caller's arrays, the arrays of a larger call from the device.
+int deliver_sim(smpm_handle* h, const smpm_sim* s) {
   const size_t n = (size_t)s->count, f = n * sizeof(float);
   size_t total = 0;
-  const size_t back = lay_out(h, n, &total);
+  lay_out(h, n, &total);
   float* dst[4] = {s->x, s->y, s->vx, s->vy};
   float* src[4] = {h->d.x, h->d.y, h->d.vx, h->d.vy};
-  char* dev = reinterpret_cast<char*>(h->d.ctrl);
-  char* host = reinterpret_cast<char*>(h->host_ctrl);
-  const bool staged = total <= h->stage_bytes;
-  cudaError_t e = cudaMemcpyAsync(host, dev, staged ? back : sizeof(Ctrl2), cudaMemcpyDeviceToHost, h->stream);
-  for (int k = 0; k < 4 && !staged; ++k) e = e ? e : cudaMemcpyAsync(dst[k], src[k], f, cudaMemcpyDeviceToHost, h->stream);
-  e = e ? e : cudaStreamSynchronize(h->stream);
-  if (e == cudaSuccess && staged && n)
-    for (int k = 0; k < 4; ++k) std::memcpy(dst[k], host + (reinterpret_cast<char*>(src[k]) - dev), f);
+  const char* dev = reinterpret_cast<char*>(h->d.ctrl);
+  const char* host = reinterpret_cast<char*>(h->host_ctrl);
+  cudaError_t e = cudaSuccess;
+  if (total <= h->stage_bytes) {
+    for (int k = 0; k < 4 && n; ++k) std::memcpy(dst[k], host + (reinterpret_cast<char*>(src[k]) - dev), f);
+  } else {
+    for (int k = 0; k < 4; ++k) e = e ? e : cudaMemcpyAsync(dst[k], src[k], f, cudaMemcpyDeviceToHost, h->stream);
+    e = e ? e : cudaStreamSynchronize(h->stream);
+  }
   if (e == cudaSuccess) h->nodes = h->host_ctrl->active_nodes;
   return h->cuda(e, "copy particles out");
+}
+
+int download_sim(smpm_handle* h, const smpm_sim* s) {
+  const int rc = fetch_sim(h, s);
+  return rc ? rc : deliver_sim(h, s);
 }
 
 int set_ctrl(smpm_handle* h, double remaining, double step) {
@@ -744,18 +781,27 @@ int smpm_frame(smpm_handle* h, const smpm_sim* s, double dt, int32_t* substeps, 
   if (rc || (rc = upload_sim(h, s, dt, 0.0))) return rc;
   const Params2 p = params_of(h, s);
   const int pb = blocks_for(s->count), gb = blocks_for(kNodes);
+  bool done = false;
   if (pb * static_cast<long long>(kThreads) >= s->count && pb <= h->frame_blocks) {
     // one particle per thread, every CTA resident: the whole frame in one launch
     Dev2 d = h->d;
     Params2 q = p;
-    void* args[] = {&d, &q};
-    cudaError_t e = cudaLaunchCooperativeKernel((const void*)k2_frame, dim3(pb), dim3(kThreads), args, 0, h->stream);
-    if ((rc = h->cuda(e, "frame launch"))) return rc;
-    if ((rc = download_sim(h, s))) return rc;
-    if (h->host_ctrl->timeout) {
-      cudaMemsetAsync(h->d.grid, 0, kNodes * sizeof(float4), h->stream);
-      return h->fail(MPM_ERR_TIMEOUT, "a bounded device wait gave up (grid barrier)");
+    Wait2 wait = h->wait;
+    void* args[] = {&d, &q, &wait};
+    if (cudaLaunchCooperativeKernel((const void*)k2_frame, dim3(pb), dim3(kThreads), args, 0, h->stream) == cudaSuccess) {
+      if ((rc = fetch_sim(h, s))) return rc;
+      done = h->host_ctrl->verdict == kFrameDone;
+      if (!done) {  // a barrier gave up: the particles are as they came, the grid holds parts of a substep
+        ++h->frames_given_up;
+        if ((rc = h->cuda(cudaMemsetAsync(h->d.grid, 0, kNodes * sizeof(float4), h->stream), "frame"))) return rc;
+        if ((rc = set_ctrl(h, dt, 0.0))) return rc;
+      }
+    } else {
+      cudaGetLastError();  // refused (too few SMs for this process, say): by launches, like a frame that gave up
     }
+  }
+  if (done) {
+    if ((rc = deliver_sim(h, s))) return rc;
     h->substeps = h->host_ctrl->steps;
     if (substeps) *substeps = h->host_ctrl->steps;
     if (advanced) *advanced = dt - h->host_ctrl->remaining;
@@ -778,6 +824,16 @@ int smpm_frame(smpm_handle* h, const smpm_sim* s, double dt, int32_t* substeps, 
   h->substeps = h->host_ctrl->steps;
   if (substeps) *substeps = h->host_ctrl->steps;
   if (advanced) *advanced = dt - h->host_ctrl->remaining;
+  return MPM_OK;
+}
+
+int smpm_check_bounded_wait(smpm_handle* h, int32_t from_barrier, int64_t polls, int64_t* frames_given_up) {
+  if (!h) return MPM_ERR_INVALID_ARG;
+  if (from_barrier < 0 || polls < 0 || polls > Wait2{}.polls)
+    return h->fail(MPM_ERR_INVALID_ARG, "from_barrier must be >= 0 and polls in [0, 2^21]");
+  if (frames_given_up) *frames_given_up = h->frames_given_up;
+  h->wait = Wait2{};
+  if (polls > 0) h->wait = Wait2{static_cast<unsigned>(from_barrier), static_cast<unsigned>(polls)};
   return MPM_OK;
 }
 

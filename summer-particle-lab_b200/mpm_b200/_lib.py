@@ -204,6 +204,7 @@ SIGNATURES = {
     "smpm_step": (ctypes.c_int, [_P, ctypes.POINTER(SmpmSim), _D]),
     "smpm_stats_get": (ctypes.c_int, [_P, ctypes.POINTER(SmpmSim), ctypes.POINTER(SmpmStats)]),
     "smpm_frame": (ctypes.c_int, [_P, ctypes.POINTER(SmpmSim), _D, ctypes.POINTER(_I32), ctypes.POINTER(_D)]),
+    "smpm_check_bounded_wait": (ctypes.c_int, [_P, _I32, _I64, ctypes.POINTER(_I64)]),
     "smpm_get_fields": (ctypes.c_int, [_P, _I64, _P]),
     "smpm_set_fields": (ctypes.c_int, [_P, _I64, _P]),
 }

@@ -370,3 +370,40 @@ def test_gpu_empty_and_invalid_calls():
     with pytest.raises(_lib.MpmError):
         m.frame(s)
     m.close()
+
+
+# a grid barrier that gives up (one poll) at the frame's start, in its middle and at its end, where some CTAs may be
+# past it: the frame is taken again in separate launches and ends as it does otherwise
+@pytest.mark.gpu
+@pytest.mark.parametrize("at", [0.0, .5, 1.0])
+def test_gpu_frame_whose_barrier_gives_up_is_taken_again(at):
+    import ctypes
+    from mpm_b200 import _lib
+
+    def sim():
+        nx, ny = 120, 100
+        s, n, rng = SolidSim(nx * ny, gravity="center"), nx * ny, np.random.default_rng(4)
+        s.count = n
+        s.x[:] = (np.tile(np.arange(nx), ny) - nx / 2) * 3.6 + rng.uniform(-.3, .3, n)
+        s.y[:] = (np.repeat(np.arange(ny), nx) - ny / 2) * 3.6 + rng.uniform(-.3, .3, n)
+        s.vx[:], s.vy[:] = rng.uniform(-20, 20, n), rng.uniform(-20, 20, n)
+        s.mass[:], s.volume[:], s.material[:] = 1.1, 1.0, 11
+        return s
+
+    s, t = sim(), sim()
+    m, ref = gpu_handle(s.capacity), gpu_handle(t.capacity)
+    given_up = ctypes.c_int64()
+    for _ in range(6):
+        steps, advanced = ref.frame(t)
+        _lib.check2(_lib.lib().smpm_check_bounded_wait(m.h, int(at * 3 * steps), 1, None), m.h)
+        n, a = m.frame(s)
+        assert n == steps and abs(a - advanced) < 1e-9
+        _lib.check2(_lib.lib().smpm_check_bounded_wait(m.h, 0, 0, ctypes.byref(given_up)), m.h)
+    if at < 1:  # at the last barrier it may also end well
+        assert given_up.value == 6
+    # two FP32 runs whose node sums are added in other orders: each within the frame tests' bound of the oracle
+    assert np.abs(s.x.astype(np.float64) - t.x).max() <= 2e-5 * EXTENT
+    assert np.abs(s.y.astype(np.float64) - t.y).max() <= 2e-5 * EXTENT
+    assert m.stats(s)["nodes"] == ref.stats(t)["nodes"]
+    m.close()
+    ref.close()
