@@ -407,3 +407,49 @@ def test_gpu_frame_whose_barrier_gives_up_is_taken_again(at):
     assert m.stats(s)["nodes"] == ref.stats(t)["nodes"]
     m.close()
     ref.close()
+
+
+# few particles on the whole grid of nodes: as many CTAs as nodes fill, most of them without a particle
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [0, 1, 130])
+def test_gpu_frame_of_few_particles_updates_every_node(n):
+    s = SolidSim(200, gravity="uniform")
+    rng = np.random.default_rng(n)
+    s.count = n
+    s.x[:n], s.y[:n] = rng.uniform(-500, 500, n), rng.uniform(-500, 500, n)
+    s.vx[:n], s.vy[:n] = rng.uniform(-20, 20, n), rng.uniform(-20, 20, n)
+    s.mass[:n], s.volume[:n], s.material[:n] = 1.1, 1.0, 11
+    t = copy_sim(s)
+    m, o = gpu_handle(200), Oracle2(200)
+    for _ in range(5):
+        ng, ag = m.frame(s)
+        nc, ac = o.frame(t)
+        assert ng == nc and abs(ag - ac) < 1e-9
+    assert np.abs(s.x[:n].astype(np.float64) - t.x[:n]).max(initial=0) <= 1e-5 * EXTENT
+    assert np.abs(s.y[:n].astype(np.float64) - t.y[:n]).max(initial=0) <= 1e-5 * EXTENT
+    assert m.stats(s)["nodes"] == o.stats(t)["nodes"]
+    m.close()
+
+
+# a frame of a few particles costs no more than a frame of a few thousand
+@pytest.mark.gpu
+def test_gpu_frame_of_few_particles_is_not_slower():
+    import time
+    took = {}
+    for n in (1, 2000):
+        s = SolidSim(n, gravity="center")
+        s.count = n
+        s.x[:], s.y[:] = (np.arange(n) % 50 - 25) * 3.6, (np.arange(n) // 50 - 25) * 3.6
+        s.mass[:], s.volume[:], s.material[:] = 1.1, 1.0, 11
+        start = [a.copy() for a in (s.x, s.y, s.vx, s.vy)]
+        m, best = gpu_handle(n), math.inf
+        for _ in range(40):
+            for a, b in zip((s.x, s.y, s.vx, s.vy), start):
+                a[:] = b
+            m.reset()
+            t0 = time.perf_counter()
+            m.frame(s)
+            best = min(best, time.perf_counter() - t0)
+        took[n] = best
+        m.close()
+    assert took[1] <= 1.5 * took[2000], took
