@@ -453,3 +453,26 @@ def test_gpu_frame_of_few_particles_is_not_slower():
         took[n] = best
         m.close()
     assert took[1] <= 1.5 * took[2000], took
+
+
+# the last counts with and without a staged copy, in one launch, and more particles than resident threads
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [65536, 65537, 160000])
+def test_gpu_frame_of_many_particles_matches_oracle(n):
+    nx, pitch, rng = 400, 2.7, np.random.default_rng(n)
+    s = SolidSim(n, gravity="center")
+    s.count = n
+    s.x[:] = (np.arange(n) % nx - nx / 2) * pitch + rng.uniform(-.2, .2, n)
+    s.y[:] = (np.arange(n) // nx - nx / 2) * pitch + rng.uniform(-.2, .2, n)
+    s.vx[:], s.vy[:] = rng.uniform(-5, 5, n), rng.uniform(-5, 5, n)
+    s.mass[:], s.volume[:], s.material[:] = 1.1, 1.0, 11
+    t = copy_sim(s)
+    m, o = gpu_handle(n), Oracle2(n)
+    for _ in range(2):
+        ng, ag = m.frame(s)
+        nc, ac = o.frame(t)
+        assert ng == nc and abs(ag - ac) < 1e-9
+    assert np.abs(s.x.astype(np.float64) - t.x).max() <= 1e-5 * EXTENT
+    assert np.abs(s.y.astype(np.float64) - t.y).max() <= 1e-5 * EXTENT
+    assert m.stats(s)["nodes"] == o.stats(t)["nodes"]
+    m.close()
