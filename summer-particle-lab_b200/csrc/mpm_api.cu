@@ -109,11 +109,13 @@ struct mpm_handle {
   mpm::RegDev rdev{};
   bool reg_dirty = true;   // domain or scenes changed since the scratch was laid out
   double reg_spacing = 0;  // spacing the scratch was laid out for
+  long long reg_fine_cells = -1;  // cells of the finer width then (-1: too many)
   // particle-pair heat exchange scratch, laid out for heat_radius
   void* hblock = nullptr;  size_t hblock_bytes = 0;
   mpm::HeatBufs hbufs{};
   mpm::HeatDev hdev{};
   double heat_radius = 0;
+  long long heat_fine_cells = -1;
   double* host_exchanged = nullptr;  // pinned readback
   int slab_planes = 0;     // batch of slabs along z: node planes shared by consecutive scenes
   // learned return mode: the network's BF16 tensor-core weights, its FP32 parameters and the gate
@@ -1088,19 +1090,35 @@ static long long layout_cells(const mpm_handle* h, double hc, std::vector<mpm::R
   return cells;
 }
 
-// The finer of two cell widths unless its cells outnumber the particles eightfold (a mostly empty grid:
-// the counts' clear and scan would cost more than the shorter candidate lists save), then the coarser;
-// the coarser decides what is refused.
-static long long choose_cells(const mpm_handle* h, double fine, double coarse, std::vector<mpm::RegScene>& rs, double* hc) {
+// When the finer of two cell widths is taken: at up to `always` cells, and up to `per_particle` for each live particle within
+// `most`. What finer cells cost is the scan of their counts, 4.6 us per million, what they save goes with the particles.
+// Regularisation, coarse and fine: 2.6 million cells for 8,000 particles 56 and 60 us, for 64,000 60 and 63, for
+// 250,000 106 and 85; 18.6 million for 1,000 59 and 143, for 600,000 190 and 234. Heat exchange, whose lists are
+// longer (both by the approximate root, 10% faster): 2.4 million for 1,000 365 and 347, for 8,000 623 and 413; 6.3 million for 1,000 235 and 236, for 64,000 363 and 292;
+// 12 million for 1,000 239 and 262, for 8,000 318 and 292, for 250,000 698 and 608.
+struct CellRule {
+  long long always, per_particle, most;
+};
+constexpr long long kMostFineCells = 1ll << 24;  // scratch of 134 MB, or that of 8 cells per particle of the capacity
+static bool takes_fine(const mpm_handle* h, const CellRule& rule, long long fine_cells) {
+  return fine_cells >= 0 && fine_cells <= std::max(rule.always, std::min(rule.per_particle * h->n, rule.most));
+}
+static CellRule reg_rule(const mpm_handle* h) { return {1 << 20, 16, std::max<long long>(kMostFineCells, 8 * h->cap)}; }
+static CellRule heat_rule(const mpm_handle* h) { return {1 << 22, 1 << 10, std::max<long long>(kMostFineCells, 8 * h->cap)}; }
+
+// The cells of one of the two widths; the coarser decides what is refused. fine_cells: how many the finer width has.
+static long long choose_cells(const mpm_handle* h, const CellRule& rule, double fine, double coarse, std::vector<mpm::RegScene>& rs,
+                              double* hc, long long* fine_cells) {
   const long long most = layout_cells(h, coarse, rs);
   *hc = coarse;
+  *fine_cells = -1;
   if (most < 0) return -1;
   std::vector<mpm::RegScene> rf;
-  const long long cells = layout_cells(h, fine, rf);
-  if (cells < 0 || cells > std::max<long long>(8 * h->cap, 1 << 20)) return most;
+  *fine_cells = layout_cells(h, fine, rf);
+  if (!takes_fine(h, rule, *fine_cells)) return most;
   rs.swap(rf);
   *hc = fine;
-  return cells;
+  return *fine_cells;
 }
 
 // Lays out the regularisation scratch for the current scenes and spacing: neighbour cells one spacing
@@ -1109,7 +1127,7 @@ static int lay_out_regularizer(mpm_handle* h) {
   const int ns = static_cast<int>(h->scenes.size());
   std::vector<mpm::RegScene> rs;
   double hc = 0;
-  const long long cells = choose_cells(h, h->reg.spacing, 2 * h->reg.spacing, rs, &hc);
+  const long long cells = choose_cells(h, reg_rule(h), h->reg.spacing, 2 * h->reg.spacing, rs, &hc, &h->reg_fine_cells);
   if (cells < 0) return fail(h, MPM_ERR_INVALID_ARG, "regularisation spacing too small for the grid");
   const int64_t cap = h->cap;
   const size_t nb = mpm::reg_scan_blocks(cells);
@@ -1157,7 +1175,8 @@ static int lay_out_regularizer(mpm_handle* h) {
 
 // The scratch for the current scenes and spacing, and the current parameters.
 static int ensure_regularizer(mpm_handle* h) {
-  if (h->reg_dirty || !h->rblock || h->reg_spacing != h->reg.spacing) {
+  if (h->reg_dirty || !h->rblock || h->reg_spacing != h->reg.spacing ||
+      takes_fine(h, reg_rule(h), h->reg_fine_cells) != (h->rdev.cells == h->reg_fine_cells)) {
     const int rc = lay_out_regularizer(h);
     if (rc != MPM_OK) return rc;
   }
@@ -1453,11 +1472,13 @@ int mpm_regularize(mpm_handle* h, double dt) {
 
 // Lays out the heat-exchange scratch for cells half a radius (or one, see choose_cells) wide over each scene's grid.
 static int ensure_heat(mpm_handle* h, double radius) {
-  if (h->hblock && h->heat_radius == radius) return MPM_OK;
+  if (h->hblock && h->heat_radius == radius &&
+      takes_fine(h, heat_rule(h), h->heat_fine_cells) == (h->hdev.cells == h->heat_fine_cells))
+    return MPM_OK;
   const int ns = static_cast<int>(h->scenes.size());
   std::vector<mpm::RegScene> rs;
   double hc = 0;
-  const long long cells = choose_cells(h, radius / 2, radius, rs, &hc);
+  const long long cells = choose_cells(h, heat_rule(h), radius / 2, radius, rs, &hc, &h->heat_fine_cells);
   if (cells < 0) return fail(h, MPM_ERR_INVALID_ARG, "heat-exchange radius too small for the grid");
   const int64_t cap = h->cap;
   const size_t nb = mpm::reg_scan_blocks(cells);

@@ -254,3 +254,51 @@ def test_lists_follow_a_body_on_grids_of_many_tiles(grid, cells_per_step):
     assert np.max(np.abs(out["F"] - st.F)) <= 2e-6 * 40 * cells_per_step
     assert sol.status() == 0
     sol.close()
+
+
+def test_pair_cells_follow_the_particle_count():
+    """One handle with few, many and few particles again: the neighbour cells are the coarse ones, the fine ones and
+    the coarse ones of a grid with 1.5 million (regularisation) and 4.9 million (heat exchange) fine cells."""
+    d = Domain(lower=(-64, -48, -64), upper=(64, 72, 64), H=8.0)
+    mats = [Material(model=0, mu=.4, lam=.4, specific_heat=cp, conductivity=k) for cp, k in ((4180.0, .6), (450.0, 80.0))]
+    spacing, radius = 1.39, 1.9
+    kw = dict(spacing=spacing, volume_unit=1.0, max_speed=8.0, rate=40.0)
+    sol = Solver(d, 100000)
+    for n in (1000, 100000, 1000):
+        rng = np.random.default_rng(n)
+        x = rng.uniform(-.5, .5, (n, 3)) * 1.1 * n ** (1 / 3)
+        sc = scenes._scene("pairs", d, mats, x, (0, 0, 0))
+        sc.m, sc.V = rng.uniform(.5, 2.0, n), rng.uniform(.5, 1.5, n)
+        sc.mat = (rng.uniform(0, 1, n) < .4).astype(np.int32)
+        sc.T = rng.uniform(20, 300, n)
+        sol.upload(sc)
+        st = orc.state_from_scene(sc)
+        st.init_enthalpy()
+        sol.exchange_heat(1 / 60, radius)
+        st.exchange_heat(1 / 60, radius=radius)
+        assert np.max(np.abs(sol.download(("T",))["T"] - st.T)) <= 1e-4 * 300  # as in test_pair_cells
+        sol.set_regularizer(True, **kw)
+        sol.regularize(1 / 240)
+        st.regularize(1 / 240, **kw)
+        assert np.max(np.abs(sol.download(("x",))["x"] - st.x)) <= d.H / 2 ** 22 + 8 / 240 * 4e-6
+    sol.close()
+
+
+def test_a_pair_pass_costs_by_its_particles_not_the_capacity():
+    import time
+    d = Domain(lower=(0, 0, 0), upper=(1, 1, 1), H=1 / 128)
+    x = scenes.block_particles(d, (4, 4, 4), (9, 9, 9), 1)
+    sc = scenes._scene("small", d, [Material.from_young(0, 1e5, .3, density=1000.0)], x, (0, 0, 0))
+    took = {}
+    for capacity in (sc.n, 4000000):
+        sol = Solver(d, capacity)
+        sol.upload(sc)
+        sol.set_regularizer(True, spacing=d.H / 2, volume_unit=(d.H / 2) ** 3, max_speed=8.0, rate=40.0)
+        times = []
+        for _ in range(20):
+            t0 = time.perf_counter()
+            sol.regularize(1e-6)
+            times.append(time.perf_counter() - t0)
+        took[capacity] = min(times)
+        sol.close()
+    assert took[4000000] <= 1.5 * took[sc.n], took
