@@ -248,6 +248,9 @@ int mpm_profile_enable(mpm_handle* h, int32_t on);
 int mpm_profile_read(mpm_handle* h, double ms[MPM_PROFILE_KERNELS], int64_t launches[MPM_PROFILE_KERNELS]);
 /* number of kernels this handle has launched (all kinds) */
 int mpm_launch_count(mpm_handle* h, int64_t* count);
+/* number of tile sorts since the handle's grid was set up: one when a state is first scattered, before each
+ * permutation of the state, and whenever particles have left the tiles of the list that the passes keep */
+int mpm_sort_count(mpm_handle* h, int64_t* count);
 
 /* ---- rollback and checkpoint (gpu/mixed_solver.py:453-480 keeps in-memory rollback copies) ---- */
 int mpm_snapshot(mpm_handle* h);

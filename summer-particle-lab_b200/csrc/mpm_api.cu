@@ -1735,6 +1735,14 @@ int mpm_launch_count(mpm_handle* h, int64_t* count) {
   return MPM_OK;
 }
 
+int mpm_sort_count(mpm_handle* h, int64_t* count) {
+  if (!h || !count) return MPM_ERR_INVALID_ARG;
+  MPM_CUDA(h, cudaMemcpyAsync(h->host_ctrl, h->ctx.ctrl, sizeof(mpm::Ctrl), cudaMemcpyDeviceToHost, h->stream));
+  MPM_CUDA(h, cudaStreamSynchronize(h->stream));
+  *count = h->host_ctrl->sorts;
+  return MPM_OK;
+}
+
 int mpm_ledger_compute(mpm_handle* h, mpm_ledger* out) {
   if (!h || !out) return MPM_ERR_INVALID_ARG;
   if (!h->uploaded) return fail(h, MPM_ERR_STATE, "no particles uploaded");

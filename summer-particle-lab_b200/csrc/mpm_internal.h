@@ -93,6 +93,7 @@ struct Ctrl {
   unsigned strays;       // particles that left the tile whose list holds them, as of the last scatter pass
   unsigned far_strays;   // some of them may leave the windows next (kFlagFar), moving fast (kFlagFast)
   unsigned first_speed;  // the largest particle speed, in cells per second (float bits), of a P2G pass's state
+  unsigned sorts;        // work lists made so far
   unsigned list_age;     // substeps since the state was last sorted (0: every particle is listed in its own tile)
   unsigned in_place;     // perm is the identity: the state was permuted after the newest sort
   unsigned last_substep; // 1 when the current substep is the call's last (set by k_open): only then

@@ -429,6 +429,7 @@ __device__ __forceinline__ void scan_tiles(const Ctx& c, int block, int blocks) 
     c.ctrl->work_count[list] = items;
     c.ctrl->sort_list = list;
     c.ctrl->in_place = 0u;
+    c.ctrl->sorts += 1u;
   };
   if (threadIdx.x == kScanThreads - 1) {  // block totals
     c.s.block_off[block] = blocks > 1 ? run.x : 0u;

@@ -150,6 +150,7 @@ SIGNATURES = {
     "mpm_profile_enable": (ctypes.c_int, [_P, _I32]),
     "mpm_profile_read": (ctypes.c_int, [_P, ctypes.POINTER(_D), ctypes.POINTER(_I64)]),
     "mpm_launch_count": (ctypes.c_int, [_P, ctypes.POINTER(_I64)]),
+    "mpm_sort_count": (ctypes.c_int, [_P, ctypes.POINTER(_I64)]),
     "mpm_ledger_compute": (ctypes.c_int, [_P, ctypes.POINTER(MpmLedger)]),
     "mpm_min_j": (ctypes.c_int, [_P, ctypes.POINTER(_D)]),
     "mpm_status": (ctypes.c_int, [_P, ctypes.POINTER(ctypes.c_uint32)]),

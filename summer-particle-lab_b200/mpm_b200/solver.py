@@ -227,6 +227,11 @@ class Solver:
         self._check(_lib.lib().mpm_launch_count(self.h, ctypes.byref(c)))
         return c.value
 
+    def sort_count(self):
+        c = ctypes.c_int64()
+        self._check(_lib.lib().mpm_sort_count(self.h, ctypes.byref(c)))
+        return c.value
+
     def stream(self):
         s = _P()
         self._check(_lib.lib().mpm_get_stream(self.h, ctypes.byref(s)))

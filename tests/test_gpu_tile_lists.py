@@ -302,3 +302,102 @@ def test_a_pair_pass_costs_by_its_particles_not_the_capacity():
         took[capacity] = min(times)
         sol.close()
     assert took[4000000] <= 1.5 * took[sc.n], took
+
+
+# the kinds of pass beside the plain one, each with lists that particles leave: conduction (which also reads node
+# temperatures outside the window), pinned particles in the lists, the window without TMA, a history law, and the
+# Newton-gated and learned returns with a body that yields
+@pytest.mark.parametrize("kind", ["conduction", "pinned", "plain loads", "sand", "newton", "learned"])
+@pytest.mark.parametrize("cells_per_step", [.04, .3, .8])
+def test_kept_lists_in_every_kind_of_pass(kind, cells_per_step, monkeypatch):
+    d = Domain(lower=(0, 0, 0), upper=(1, 1, 1), H=1 / 32)
+    yields = kind in ("newton", "learned")
+    dt, steps = 1e-6 if yields else 1e-5, 14
+    v = cells_per_step * d.H / dt
+    x = scenes.block_particles(d, (3, 3, 3), (10, 8, 9), 5)
+    mat = Material.from_young(0, 1e5, .3, density=1000.0, specific_heat=1000.0)
+    if yields:
+        mat = scenes.johnson_cook_metal(7)
+    if kind == "sand":
+        mat = Material.reference_units(3, E=1e5, density=1000.0)
+    if kind == "pinned":  # a fixed block three cells beside the moving one's path, in the same tiles
+        x = np.concatenate([x, scenes.block_particles(d, (3, 3, 13), (12, 8, 15), 6)])
+    sc = scenes._scene(kind, d, [mat], x, (v, 0, 0))
+    if kind == "pinned":
+        sc.pinned = (x[:, 2] > 11 * d.H).astype(np.uint8)
+        sc.v[sc.pinned == 1] = 0
+    if kind == "conduction":
+        sc.T = np.where(x[:, 0] < 6.5 * d.H, 400.0, 300.0)
+        sc.meta["conduction"] = dict(k=5e5, rho=1000.0, cp=1000.0)
+    if yields:
+        sc.F = np.tile((np.eye(3) + np.diag([.008, -.004, -.004])).ravel(), (sc.n, 1))
+    if kind == "plain loads":
+        monkeypatch.setenv("MPM_B200_NO_TMA", "1")
+    sol = Solver(d, sc.n)
+    sol.upload(sc)
+    if kind == "newton":
+        sol.set_return_mode(mode="newton", gate_tol=1e-5, newton=8)
+    if kind == "learned":
+        from mpm_b200.surrogate import Surrogate
+        net = Surrogate(mat, seed=3)
+        sol.set_return_mode(net, gate_tol=1e-5, newton=4)
+        net.close()
+    st = orc.state_from_scene(sc)
+    sol.step_fixed(dt, steps)
+    for _ in range(steps):
+        st.step(dt)
+    out = sol.download(("x", "F", "T", "ep"))
+    assert sol.status() == 0
+    # the bounds of the moving body above; temperatures and plastic strain as in their own tests
+    assert np.max(np.abs(out["x"] - st.x)) <= 1e-6 + steps * d.H / 2 ** 23 + 4 * steps * dt * v * 2.0 ** -24
+    assert np.max(np.abs(out["F"] - st.F)) <= 2e-6 * max(1.0, 40 * cells_per_step)
+    if kind == "conduction":
+        assert np.max(np.abs(out["T"] - st.T)) <= 1e-5 * 100
+    if yields:
+        assert np.max(st.ep) > 0
+        assert np.max(np.abs(out["ep"] - st.ep)) <= 2e-6 + 1e-4 * np.max(st.ep)
+    sol.close()
+
+
+# a batch whose one fast scene holds too few of its particles to bring a sort by their share, eagerly and in a graph
+@pytest.mark.parametrize("graph", [False, True])
+def test_kept_lists_of_a_batch_with_one_fast_scene(graph):
+    from mpm_b200.solver import Batch
+    subs, steps = [], 72
+    for k in range(3):
+        d = Domain(lower=(0, 0, 0), upper=(1, 1, 1), H=1 / 48)
+        fast = k == 1
+        x = scenes.block_particles(d, (3, 3, 3), (5, 5, 5) if fast else (13, 13, 13), 60 + k)
+        subs.append(scenes._scene("s%d" % k, d, [Material.from_young(0, 1e5, .3, density=1000.0)], x, (240.0 if fast else .5, 0, 0)))
+    b = Batch(subs)
+    b.upload()
+    b.run(steps, graph=graph)
+    parts, times = b.split(b.download(("x", "F"))), b.times()[0]
+    assert b.status() == 0
+    b.close()
+    for k, sc in enumerate(subs):
+        st, t = orc.state_from_scene(sc), 0.0
+        for _ in range(steps):
+            dt = st.stable_dt()
+            st.step(dt)
+            t += dt
+        far = abs(sc.v[0, 0]) * t
+        # the time follows from FP32 maxima (four roundings of 2^-24 a substep at most); positions as above
+        assert abs(times[k] - t) <= 4 * 2.0 ** -24 * t * steps ** .5 + 1e-6 * t
+        assert np.max(np.abs(parts[k]["x"] - st.x)) <= 1e-6 + steps * sc.domain.H / 2 ** 23 + 8 * 2.0 ** -24 * far + 2e-6 * far
+        assert np.max(np.abs(parts[k]["F"] - st.F)) <= 2e-6 * 16
+
+
+# sorts in 24 substeps beside the first scatter's: none while a body stays, at most every other substep while lists last two of
+# them, every one past half a cell
+@pytest.mark.parametrize("cells_per_step,least,most", [(0.0, 0, 0), (.0004, 0, 0), (.3, 8, 13), (.8, 22, 24)])
+def test_sorts_follow_the_motion(cells_per_step, least, most):
+    d = Domain(lower=(0, 0, 0), upper=(1, 1, 1), H=1 / 64)
+    x = scenes.block_particles(d, (2, 2, 2), (12, 8, 9), 5)
+    dt = 1e-6
+    sc = scenes._scene("moving", d, [Material.from_young(0, 1e5, .3, density=1000.0)], x, (cells_per_step * d.H / dt, 0, 0))
+    sol = Solver(d, sc.n)
+    sol.upload(sc)
+    sol.step_fixed(dt, 24)
+    assert least <= sol.sort_count() - 1 <= most
+    sol.close()
