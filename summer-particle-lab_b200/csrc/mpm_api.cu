@@ -468,13 +468,20 @@ static int check_status(mpm_handle* h) {
 }
 
 // Particles per work item of the particle pass, as a power of two (31: whole tiles). A tile costs a CTA about
-// 9 us whatever it holds, so tiles are split only while the parts still find CTAs of their own: 256
-// particles (one round of phase A) up to as many as the resident CTAs hold at that size. Substep at 13,824
-// particles 33.1 -> 27.8 us, at 45,448 34.1 -> 29.9, at 131,072 47.5 -> 48.9 (so not split). The history laws' long
-// phase A moves the line: 171,360 particles of soil 81.9 -> 77.5 us.
+// 9 us whatever it holds, so tiles are split, into parts of 256 particles (one round of phase A), only where that fills
+// CTAs that would idle: while the parts find a CTA each, and, with the history laws' longer phase A, where whole tiles
+// would leave most of a second round empty. By the particles over those of as many full tiles as CTAs are
+// resident (151,552); substep with whole tiles and with parts, particles at rest and at .02 cells a substep:
+//   0.34  J2 31.7 and 29.2, 35.6 and 31.0 us; sand 35.6 and 31.6, 42.6 and 34.1
+//   0.42  J2 31.6 and 35.6, 37.3 and 39.1;    sand 36.0 and 39.9, 44.3 and 44.8
+//   0.73  J2 34.3 and 35.7, 39.2 and 43.2;    sand 39.0 and 40.3, 46.5 and 50.3
+//   0.93  J2 45.8 and 44.1, 50.7 and 50.2;    sand 53.3 and 50.9, 61.2 and 58.2
+//   1.16                                      sand 53.3 and 50.8, 65.5 and 64.4
+//   1.43                                      sand 56.1 and 61.4, 67.9 and 71.7
+// Snow and foam lie beside sand, fixed-corotated and Johnson-Cook beside J2.
 static int split_shift(const mpm_handle* h) {
-  const int64_t resident = static_cast<int64_t>(h->p2g_blocks) << kMinSplitShift;
-  return h->n <= resident * (h->ctx.has_aux ? 3 : 1) ? kMinSplitShift : 31;
+  const double full = static_cast<double>(h->n) / (512.0 * std::max(1, h->p2g_blocks));
+  return full <= 0.375 || (h->ctx.has_aux && full > 0.75 && full <= 1.25) ? kMinSplitShift : 31;
 }
 
 // Counting sort of the current state by tile and the dt-free P2G into acc[step_index & 1].

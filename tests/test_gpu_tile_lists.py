@@ -401,3 +401,9 @@ def test_sorts_follow_the_motion(cells_per_step, least, most):
     sol.step_fixed(dt, 24)
     assert least <= sol.sort_count() - 1 <= most
     sol.close()
+
+
+# whole tiles and parts on both sides of the rule's lines, of 56,832, 113,664 and 189,440 particles on 148 SMs
+@pytest.mark.parametrize("n,model", [(56832, 0), (56833, 0), (113664, 3), (113665, 3), (189441, 3)])
+def test_tile_parts_on_both_sides_of_their_lines(n, model):
+    test_tile_counts(n, 12, model)
