@@ -297,7 +297,6 @@ static void finish_sort(mpm_handle* h) {
 }
 
 // Permutation pass: rewrite the state in sort order into the other buffer and make it current.
-
 static int permute_state(mpm_handle* h) {
   finish_sort(h);
   h->ctx.n = h->n;
@@ -1097,12 +1096,12 @@ static long long layout_cells(const mpm_handle* h, double hc, std::vector<mpm::R
   return cells;
 }
 
-// When the finer of two cell widths is taken: at up to `always` cells, and up to `per_particle` for each live particle within
-// `most`. What finer cells cost is the scan of their counts, 4.6 us per million, what they save goes with the particles.
+// When the finer of two cell widths is taken: at up to `always` cells, and up to `per_particle` for each live particle
+// within `most`. What finer cells cost is the scan of their counts, 4.6 us per million, what they save goes with the particles.
 // Regularisation, coarse and fine: 2.6 million cells for 8,000 particles 56 and 60 us, for 64,000 60 and 63, for
 // 250,000 106 and 85; 18.6 million for 1,000 59 and 143, for 600,000 190 and 234. Heat exchange, whose lists are
-// longer (both by the approximate root, 10% faster): 2.4 million for 1,000 365 and 347, for 8,000 623 and 413; 6.3 million for 1,000 235 and 236, for 64,000 363 and 292;
-// 12 million for 1,000 239 and 262, for 8,000 318 and 292, for 250,000 698 and 608.
+// longer (both by the approximate root, 10% faster): 2.4 million for 1,000 365 and 347, for 8,000 623 and 413; 6.3
+// million for 1,000 235 and 236, for 64,000 363 and 292; 12 million for 1,000 239 and 262, for 8,000 318 and 292, for 250,000 698 and 608.
 struct CellRule {
   long long always, per_particle, most;
 };

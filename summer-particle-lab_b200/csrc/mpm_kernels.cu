@@ -1,8 +1,8 @@
 // CUDA kernels of the B200-native MLS-MPM solid step (sm_100a).
 //
 // One substep is three launches on one stream (no host sync):
-//   k_open         1 CTA: dt from the device-side CFL maxima, step bookkeeping, list resets; after a pass
-//                  that wrote sort keys, the scan of the tile counts
+//   k_open         one CTA: dt from the device-side CFL maxima, step bookkeeping, list resets; the others, after a
+//                  pass that wrote sort keys: the scan of the tile counts, 4,096 tiles each
 //   k_grid_sort    active node tiles only: v = (p + dt (f + m g)) / m, walls, sticky floor; beside it, after
 //                  such a pass, the counting sort: perm[start + rank] = particle
 //   k_particles    per particle tile: TMA-staged 8^3 velocity window -> gather v, C -> F update
@@ -302,7 +302,7 @@ __device__ __forceinline__ void begin_substep(const Ctx& c) {
       ct->substeps += 1;
       ct->step_substeps += 1;
       ct->advanced += dt;
-      // the next k_begin ends the call after this substep (the same tests it will make)
+      // the next opening ends the call after this substep (the same tests it will make)
       bool last;
       if (ct->mode == kModeRequested)
         last = ct->steps_left <= 1 &&
@@ -1232,8 +1232,6 @@ __device__ __forceinline__ unsigned particle_phase_a(const Ctx& c, const SceneDe
     }
     if (in_w && !pinned) {
       const int bucket = (l2 * 6 + l1) * 6 + l0;
-      // one shared atomic per bucket among the warp's converged lanes (particles of one cell share
-      // buckets), each lane's rank from its position among them
       // one shared integer atomic per particle: grouping the warp's lanes by bucket first
       // (__match_any_sync) took 2% longer
       const int rank = atomicAdd(&hist[bucket], 1);
@@ -1570,7 +1568,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_particles(const __grid_constant__
   if (PASS != kPassP2G && ct->done) return;
   const unsigned k = ct->step_index;
   const bool store_vc = ct->last_substep != 0u;
-  const int nxt = k & 1;  // the pass scatters into acc[k & 1] (k_begin advanced k before a substep)
+  const int nxt = k & 1;  // the pass scatters into acc[k & 1] (k_open advanced k before a substep)
   const bool use_tma = GATHER && c.use_tma;
   const bool single = c.single_material != 0 || c.scene_material != 0;
 

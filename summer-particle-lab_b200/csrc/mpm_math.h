@@ -684,8 +684,8 @@ MPM_NOINLINE ConstitutiveOut constitutive_pressure(const MaterialDev& mt, const 
   return out;
 }
 
-// exp(x) - 1 for |x| <= 0.26 (on the series path |tr L| stays below 0.15) by its Taylor series to x^8:
-// truncation below 2e-11 of the result.
+// exp(x) - 1 for |x| <= 0.26 (on the series path |tr L| stays below 0.15) by its Taylor series to x^8: the next
+// term is x^8 / 9! of the result, 6e-11 at 0.26 and under 1e-12 at 0.15.
 MPM_HD float expm1_small(float x) {
   float p = 1.f / 40320.f;
   p = fmaf(p, x, 1.f / 5040.f);

@@ -11,7 +11,8 @@
 //                  (position, target, inverse mass, index, material) in cell order, so neighbour
 //                  candidates are read as contiguous runs
 //   k_reg_pairs    thread per particle in cell order: its own shift, gathered over the rows of cells
-//                  within half the sum of its own and the scene's largest target (ball_rows). The reference visits each pair once (i < j) and adds +shift to i and -shift to j; the pair
+//                  within half the sum of its own and the scene's largest target (ball_rows). The
+//                  reference visits each pair once (i < j) and adds +shift to i and -shift to j; the pair
 //                  term is antisymmetric, so gathering every neighbour from each side gives the
 //                  same sums without atomics. The largest shift of each scene over its budget.
 //   k_reg_apply    x += shift / max(1, largest / budget) for unpinned particles, clamped to the box

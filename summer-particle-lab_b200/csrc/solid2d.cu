@@ -9,10 +9,11 @@
 //     one float4 vector atomic per node per particle. The grid pass normalises, applies the
 //     walls, writes node velocities and clears the accumulator in the same read, so no
 //     separate clear launch exists.
-//   * smpm_frame runs the whole MPM branch of Simulation.step on the device: G2P fuses the
-//     next substep's stableStep reduction, and the last block to finish decides the next
-//     substep length and whether the frame is done, so the host launches batches of substeps
-//     and reads one small control block per batch.
+//   * smpm_frame runs the whole MPM branch of Simulation.step on the device, in one cooperative launch for as
+//     many particles as threads are resident (k2_frame). Beyond them, or where that launch is refused or a barrier
+//     gives up, in launches per substep: G2P fuses the next substep's stableStep reduction, and the last
+//     block to finish decides the next substep length and whether the frame is done, so the host launches
+//     batches of substeps and reads one small control block per batch.
 #include <cuda_runtime.h>
 
 #include <algorithm>
