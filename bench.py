@@ -267,7 +267,7 @@ class Clocks:
 # one ncu --set full capture of k_particles<1,0,0> on the 2M-particle J2 drop, divided by the particle
 # count), set by hand from that capture; bench.py scales it to the timed workload's particle count.
 TRAFFIC_PER_PARTICLE = 146.0
-TRAFFIC_SOURCE = "ncu --set full capture of k_particles<1,0,0,0>, j2_drop 2,097,152 particles (306.1 MB per launch)"
+TRAFFIC_SOURCE = "ncu --set full capture of k_particles<1,0,0,0>, j2_drop 2,097,152 particles (306.2 MB per launch)"
 
 
 def peaks():
